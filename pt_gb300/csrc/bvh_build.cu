@@ -944,8 +944,11 @@ size_t bvh_node_count(uint32_t tri_count, uint32_t instance_count)
 // (|x| > 65504) rounds to an infinity; the node stays conservative, but
 // `*overflow` is set so that the caller traverses the BVH2 instead (an
 // infinite plane times the infinite inverse direction of an axis-parallel ray
-// gives NaN slab distances).  Slots of the node array that no tree uses hold
-// zeros (the caller clears the array before the build); the bounds check
+// gives NaN slab distances).  An unused child slot holds planes that no ray
+// with a finite inverse direction meets (x planes at +inf, y planes at -inf: a
+// ray that goes toward both has its z exit before the infinite entry), so the
+// traversal need not compare the links.  Slots of the node array that no tree
+// uses hold zeros (the caller clears the array before the build); the bounds check
 // keeps their derivation inside the array.
 __global__ void k_make_bvh4(const BvhNode* nodes, uint32_t n, Bvh4Node* out, uint32_t* overflow)
 {
@@ -980,7 +983,7 @@ __global__ void k_make_bvh4(const BvhNode* nodes, uint32_t n, Bvh4Node* out, uin
     }
     for (; k < 4; k++) {
         for (int a = 0; a < 6; a++)
-            b[a][k] = 0.0f;
+            b[a][k] = a < 2 ? __int_as_float(0x7f800000) : a < 4 ? __int_as_float(0xff800000) : 0.0f;
         ref[k] = REF_EMPTY;
     }
     Bvh4Node o;
@@ -991,7 +994,7 @@ __global__ void k_make_bvh4(const BvhNode* nodes, uint32_t n, Bvh4Node* out, uin
             const __half h0 = (a & 1) ? __float2half_ru(b[a][2 * j]) : __float2half_rd(b[a][2 * j]);
             const __half h1 = (a & 1) ? __float2half_ru(b[a][2 * j + 1]) : __float2half_rd(b[a][2 * j + 1]);
             q[a][j] = (uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16);
-            if (__hisinf(h0) || __hisinf(h1))
+            if ((__hisinf(h0) && ref[2 * j] != REF_EMPTY) || (__hisinf(h1) && ref[2 * j + 1] != REF_EMPTY))
                 *overflow = 1u;
         }
     }

@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 
 #include "ptmath.cuh"
+#include "slab.h"
 
 namespace pt {
 
@@ -231,14 +232,26 @@ struct Ray {
 struct ObjRay {
     f3 o, d;
     f3 inv_d, o_inv; // 1/d and o/d for the slab test
-    int kx, ky, kz;
+    uint32_t axes;   // SLAB_HI_*: the planes met first; AXIS_*: the permutation of the watertight test
     float sx, sy, sz;
 };
+
+// ObjRay::axes.  SLAB_HI_*: the upper plane of that slab is met first (slab.h).
+constexpr uint32_t SLAB_HI_X = 1u, SLAB_HI_Y = 2u, SLAB_HI_Z = 4u;
+constexpr uint32_t AXIS_X_IS_1 = 8u, AXIS_X_IS_2 = 16u, AXIS_Y_IS_1 = 32u, AXIS_Y_IS_2 = 64u, AXIS_Z_IS_1 = 128u, AXIS_Z_IS_2 = 256u;
 
 __device__ __forceinline__ void setup_slab(ObjRay& r)
 {
     r.inv_d = mk3(1.0f / r.d.x, 1.0f / r.d.y, 1.0f / r.d.z);
     r.o_inv = mk3(r.o.x * r.inv_d.x, r.o.y * r.inv_d.y, r.o.z * r.inv_d.z);
+    r.axes = (slab_hi_first(__float_as_uint(r.inv_d.x)) ? SLAB_HI_X : 0u) | (slab_hi_first(__float_as_uint(r.inv_d.y)) ? SLAB_HI_Y : 0u) |
+             (slab_hi_first(__float_as_uint(r.inv_d.z)) ? SLAB_HI_Z : 0u);
+}
+
+// Component of v along a permuted axis of the ray (is1, is2: its AXIS_ bits).
+__device__ __forceinline__ float along(f3 v, uint32_t axes, uint32_t is1, uint32_t is2)
+{
+    return (axes & is2) ? v.z : (axes & is1) ? v.y : v.x;
 }
 
 __device__ __forceinline__ void setup_watertight(ObjRay& r)
@@ -257,9 +270,8 @@ __device__ __forceinline__ void setup_watertight(ObjRay& r)
         kx = ky;
         ky = t;
     }
-    r.kx = kx;
-    r.ky = ky;
-    r.kz = kz;
+    r.axes |= (kx == 1 ? AXIS_X_IS_1 : 0u) | (kx == 2 ? AXIS_X_IS_2 : 0u) | (ky == 1 ? AXIS_Y_IS_1 : 0u) |
+              (ky == 2 ? AXIS_Y_IS_2 : 0u) | (kz == 1 ? AXIS_Z_IS_1 : 0u) | (kz == 2 ? AXIS_Z_IS_2 : 0u);
     r.sx = comp(r.d, kx) / dz;
     r.sy = comp(r.d, ky) / dz;
     r.sz = 1.0f / dz;
@@ -319,47 +331,77 @@ __device__ __forceinline__ float fmax3f(float a, float b, float c)
     return d;
 }
 
-// One axis of a half-precision 4-wide node: the lower and upper planes of the
-// four children as floats (exact: every half is a float).
-__device__ __forceinline__ void unpack_planes(const uint4& q, float4& lo, float4& hi)
+// One axis of a half-precision 4-wide node: the planes of the four children
+// that the ray meets first and last, as floats (exact: every half is a float).
+__device__ __forceinline__ void unpack_planes(const uint4& q, bool hi_first, float4& first, float4& last)
 {
-    const float2 l01 = __half22float2(*reinterpret_cast<const __half2*>(&q.x));
-    const float2 l23 = __half22float2(*reinterpret_cast<const __half2*>(&q.y));
-    const float2 h01 = __half22float2(*reinterpret_cast<const __half2*>(&q.z));
-    const float2 h23 = __half22float2(*reinterpret_cast<const __half2*>(&q.w));
-    lo = make_float4(l01.x, l01.y, l23.x, l23.y);
-    hi = make_float4(h01.x, h01.y, h23.x, h23.y);
+    const uint32_t f0 = hi_first ? q.z : q.x, f1 = hi_first ? q.w : q.y, l0 = hi_first ? q.x : q.z, l1 = hi_first ? q.y : q.w;
+    const float2 f01 = __half22float2(*reinterpret_cast<const __half2*>(&f0));
+    const float2 f23 = __half22float2(*reinterpret_cast<const __half2*>(&f1));
+    const float2 l01 = __half22float2(*reinterpret_cast<const __half2*>(&l0));
+    const float2 l23 = __half22float2(*reinterpret_cast<const __half2*>(&l1));
+    first = make_float4(f01.x, f01.y, f23.x, f23.y);
+    last = make_float4(l01.x, l01.y, l23.x, l23.y);
+}
+
+// A 4-wide node by two 32-byte loads (sm_100 and later).  ptxas of CUDA 13.0
+// crashes on them in the megakernel's out-of-line traversal, whose translation
+// unit defines PT_NARROW_NODE_LOADS.  Heavy scene: 28.9 -> 28.4 ms of extend,
+// the mid scene unchanged.
+__device__ __forceinline__ void load_node4(const Bvh4Node* node, uint4& qx, uint4& qy, uint4& qz, int4& l)
+{
+#ifdef PT_NARROW_NODE_LOADS
+    qx = __ldg(&node->x);
+    qy = __ldg(&node->y);
+    qz = __ldg(&node->z);
+    l = ldg4i(&node->link);
+#else
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(qx.x), "=r"(qx.y), "=r"(qx.z), "=r"(qx.w), "=r"(qy.x), "=r"(qy.y), "=r"(qy.z), "=r"(qy.w)
+        : "l"(&node->x));
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(qz.x), "=r"(qz.y), "=r"(qz.z), "=r"(qz.w), "=r"(l.x), "=r"(l.y), "=r"(l.z), "=r"(l.w)
+        : "l"(&node->z));
+#endif
 }
 
 // Intersect the four child boxes of a 4-wide node; bit k of the result is
 // set when child k is hit, e[k] its entry distance.  The boxes contain the
 // BVH2's (outward rounding), so a child the BVH2 would enter is entered here
-// too and the closest hit is the same.  The far distance is
+// too and the closest hit is the same.  The ray's direction signs say which
+// plane of a slab is met first, so that entry and exit take one distance each
+// (a select per packed pair of planes) instead of the minimum and maximum of
+// both: the kernel is bound by its issue slots (70 % busy, the pipe that
+// selects and compares 50 %), and with this and the unused slots below the
+// extend stage of the mid scene at 1024 x 1024, 128 spp went from 69.7 to
+// 58.7 ms, on the heavy scene at 1920 x 1080, 4 spp from 28.9 to 24.5.  The
+// multiply-adds as packed pairs (fma.rn.f32x2) gained nothing (59.3 ms).  The exit distance is
 // scaled once after the minimum over the axes instead of once per axis:
-// rounding is monotonic, so min(a s, b s, c s) = min(a, b, c) s for s > 0 and
-// the value equals the per-axis form of slab_enter bit for bit.
+// rounding is monotonic, so min(a s, b s, c s) = min(a, b, c) s for s > 0.
+// An unused slot (REF_EMPTY) has planes that no finite ray meets
+// (k_make_bvh4); a ray that enters it all the same finds nothing there.
 __device__ __forceinline__ int node4_children(const Bvh4Node* node, const ObjRay& r, float tmin, float tmax, float (&e)[4], int (&c)[4])
 {
-    const uint4 qx = __ldg(&node->x), qy = __ldg(&node->y), qz = __ldg(&node->z);
-    float4 lx, hx, ly, hy, lz, hz;
-    unpack_planes(qx, lx, hx);
-    unpack_planes(qy, ly, hy);
-    unpack_planes(qz, lz, hz);
-    const int4 l = ldg4i(&node->link);
+    uint4 qx, qy, qz;
+    int4 l;
+    load_node4(node, qx, qy, qz, l);
+    float4 nx, fx, ny, fy, nz, fz;
+    unpack_planes(qx, (r.axes & SLAB_HI_X) != 0, nx, fx);
+    unpack_planes(qy, (r.axes & SLAB_HI_Y) != 0, ny, fy);
+    unpack_planes(qz, (r.axes & SLAB_HI_Z) != 0, nz, fz);
     c[0] = l.x;
     c[1] = l.y;
     c[2] = l.z;
     c[3] = l.w;
     int m = 0;
-#define PT_NODE4_CHILD(k, q)                                                                     \
-    {                                                                                            \
-        const float x0 = fmaf(lx.q, r.inv_d.x, -r.o_inv.x), x1 = fmaf(hx.q, r.inv_d.x, -r.o_inv.x); \
-        const float y0 = fmaf(ly.q, r.inv_d.y, -r.o_inv.y), y1 = fmaf(hy.q, r.inv_d.y, -r.o_inv.y); \
-        const float z0 = fmaf(lz.q, r.inv_d.z, -r.o_inv.z), z1 = fmaf(hz.q, r.inv_d.z, -r.o_inv.z); \
-        e[k] = fmaxf(fmax3f(fminf(x0, x1), fminf(y0, y1), fminf(z0, z1)), tmin);                   \
-        const float far = fmin3f(fmaxf(x0, x1), fmaxf(y0, y1), fmaxf(z0, z1)) * SLAB_SCALE;      \
-        const float x = fminf(far, tmax);                                                        \
-        m |= (e[k] <= x && l.q != REF_EMPTY) ? (1 << k) : 0;                                     \
+#define PT_NODE4_CHILD(k, q)                                                                                                  \
+    {                                                                                                                         \
+        const float x0 = fmaf(nx.q, r.inv_d.x, -r.o_inv.x), x1 = fmaf(fx.q, r.inv_d.x, -r.o_inv.x);                           \
+        const float y0 = fmaf(ny.q, r.inv_d.y, -r.o_inv.y), y1 = fmaf(fy.q, r.inv_d.y, -r.o_inv.y);                           \
+        const float z0 = fmaf(nz.q, r.inv_d.z, -r.o_inv.z), z1 = fmaf(fz.q, r.inv_d.z, -r.o_inv.z);                           \
+        e[k] = fmaxf(fmax3f(x0, y0, z0), tmin);                                                                               \
+        const float far = fmin3f(x1, y1, z1) * SLAB_SCALE;                                                                    \
+        m |= e[k] <= fminf(far, tmax) ? (1 << k) : 0;                                                                         \
     }
     PT_NODE4_CHILD(0, x)
     PT_NODE4_CHILD(1, y)
@@ -373,39 +415,31 @@ constexpr int STACK_SIZE = 96;
 
 // One interior step of a 4-wide traversal: the nearest hit child becomes
 // `ref`, the others are pushed far to near (SORT; else in slot order, for
-// any-hit queries whose result does not depend on the order); nothing hit
-// pops the stack.  A push that would overflow sets ERR_STACK_OVERFLOW and
-// drops those children.
-template <bool SORT = true, class Stack>
-__device__ __forceinline__ void step4(const DevScene& s, const ObjRay& r, float tmin, float tmax, int& ref, Stack& stack, int& sp)
+// any-hit queries whose result does not depend on the order).  Returns false
+// when no child was hit (the caller pops).  A push that would overflow sets
+// ERR_STACK_OVERFLOW and drops those children.
+template <bool SORT, class Stack>
+__device__ __forceinline__ bool step4(const DevScene& s, const ObjRay& r, float tmin, float tmax, int& ref, Stack& stack, int& sp)
 {
-    constexpr int N = STACK_SIZE;
     float e[4];
     int c[4];
     const int m = node4_children(s.nodes4 + ref, r, tmin, tmax, e, c);
     const int cnt = __popc(m);
-    if (cnt == 0) {
-        ref = stack.get(--sp);
-        return;
-    }
+    if (cnt == 0)
+        return false;
     if (cnt == 1) {
         ref = c[__ffs(m) - 1];
-        return;
+        return true;
     }
     if (!SORT) {
-        if (sp + cnt - 1 > N) {
+        ref = c[__ffs(m) - 1];
+        if (sp + cnt - 1 > STACK_SIZE) {
             atomicOr(s.error_word, ERR_STACK_OVERFLOW);
-            ref = c[__ffs(m) - 1];
-            return;
+            return true;
         }
-        int rest = m;
-        ref = c[__ffs(rest) - 1];
-        rest &= rest - 1;
-        while (rest) {
+        for (int rest = m & (m - 1); rest; rest &= rest - 1)
             stack.set(sp++, c[__ffs(rest) - 1]);
-            rest &= rest - 1;
-        }
-        return;
+        return true;
     }
     // sort (entry, child) ascending with misses keyed +inf: a five-exchange network
     const float inf = __int_as_float(0x7f800000);
@@ -426,7 +460,7 @@ __device__ __forceinline__ void step4(const DevScene& s, const ObjRay& r, float 
     PT_CSWAP(k1, r1, k3, r3)
     PT_CSWAP(k1, r1, k2, r2)
 #undef PT_CSWAP
-    if (sp + cnt - 1 > N) {
+    if (sp + cnt - 1 > STACK_SIZE) {
         atomicOr(s.error_word, ERR_STACK_OVERFLOW);
     } else {
         if (cnt == 4)
@@ -436,15 +470,19 @@ __device__ __forceinline__ void step4(const DevScene& s, const ObjRay& r, float 
         stack.set(sp++, r1);
     }
     ref = r0;
+    return true;
 }
 
 // Watertight ray/triangle test (Woop, Benthin & Wald 2013) without culling.
 __device__ __forceinline__ bool watertight(const ObjRay& r, f3 p0, f3 p1, f3 p2, float& t, float& b1, float& b2)
 {
     f3 A = p0 - r.o, B = p1 - r.o, C = p2 - r.o;
-    float Akx = comp(A, r.kx), Aky = comp(A, r.ky), Akz = comp(A, r.kz);
-    float Bkx = comp(B, r.kx), Bky = comp(B, r.ky), Bkz = comp(B, r.kz);
-    float Ckx = comp(C, r.kx), Cky = comp(C, r.ky), Ckz = comp(C, r.kz);
+    float Akx = along(A, r.axes, AXIS_X_IS_1, AXIS_X_IS_2), Aky = along(A, r.axes, AXIS_Y_IS_1, AXIS_Y_IS_2);
+    float Akz = along(A, r.axes, AXIS_Z_IS_1, AXIS_Z_IS_2);
+    float Bkx = along(B, r.axes, AXIS_X_IS_1, AXIS_X_IS_2), Bky = along(B, r.axes, AXIS_Y_IS_1, AXIS_Y_IS_2);
+    float Bkz = along(B, r.axes, AXIS_Z_IS_1, AXIS_Z_IS_2);
+    float Ckx = along(C, r.axes, AXIS_X_IS_1, AXIS_X_IS_2), Cky = along(C, r.axes, AXIS_Y_IS_1, AXIS_Y_IS_2);
+    float Ckz = along(C, r.axes, AXIS_Z_IS_1, AXIS_Z_IS_2);
     float Ax = Akx - r.sx * Akz, Ay = Aky - r.sy * Akz;
     float Bx = Bkx - r.sx * Bkz, By = Bky - r.sy * Bkz;
     float Cx = Ckx - r.sx * Ckz, Cy = Cky - r.sy * Ckz;
@@ -502,37 +540,31 @@ __device__ __forceinline__ bool better(float t, uint32_t inst, uint32_t prim, co
 
 
 // BVH2 interior step: the nearer hit child becomes `ref`, the farther is
-// pushed; nothing hit pops the stack.
+// pushed; false when nothing is hit (the caller pops).
 template <class Stack>
-__device__ __forceinline__ void step2(const DevScene& s, const ObjRay& r, float tmin, float tmax, int& ref, Stack& stack, int& sp)
+__device__ __forceinline__ bool step2(const DevScene& s, const ObjRay& r, float tmin, float tmax, int& ref, Stack& stack, int& sp)
 {
-    constexpr int N = STACK_SIZE;
     float e0, e1;
     int c0, c1;
     const int m = node_children(s.nodes + ref, r, tmin, tmax, e0, e1, c0, c1);
+    if (m == 0)
+        return false;
     if (m == 3) {
-        int near = c0, far = c1;
-        if (e1 < e0) {
-            near = c1;
-            far = c0;
-        }
-        if (sp < N)
-            stack.set(sp++, far);
+        const bool swap = e1 < e0;
+        if (sp < STACK_SIZE)
+            stack.set(sp++, swap ? c0 : c1);
         else
             atomicOr(s.error_word, ERR_STACK_OVERFLOW);
-        ref = near;
-    } else if (m == 1) {
-        ref = c0;
-    } else if (m == 2) {
-        ref = c1;
+        ref = swap ? c1 : c0;
     } else {
-        ref = stack.get(--sp);
+        ref = m == 1 ? c0 : c1;
     }
+    return true;
 }
 
 // Closest-hit traversal of one ray as a resumable state: closest_begin sets
 // it up and each closest_step advances it by one node visit, leaf or
-// instance transition, returning true when the ray is finished.  The hit is
+// instance entry, returning true when the ray is finished.  The hit is
 // the (t, instance, primitive) minimum of the oracle whatever the BVH.  The
 // stack lives in local memory (L1-resident).  W4 walks the 4-wide nodes
 // (s.nodes4, which must be present), else the BVH2.
@@ -545,43 +577,17 @@ struct ClosestTrace {
     bool in_blas, found;
 };
 // The traversal stack is kept apart from the state: inside the state it
-// would pull every field of the state into local memory with it.  It lives in
-// local memory (L1).  Built with PT_SMEM_STACK = k > 0, its first k entries
-// live in shared memory instead, entry i of thread x at word i * 128 + x
-// (every lane in its own bank whatever its depth); that measured slower on
-// the mid scene (extend 72.0 ms per step in local memory, 77.9 with 8 entries
-// and 78.6 with 16 in shared memory: the per-access branch and the smaller
-// L1 cost more than the bank-parallel accesses save).  Every kernel that
-// traverses runs blocks of at most 128 threads; a stack is used by one
-// traversal at a time per thread.
-#ifndef PT_SMEM_STACK
-#define PT_SMEM_STACK 0
-#endif
-constexpr int STACK_SMEM = PT_SMEM_STACK;
-constexpr int STACK_BLOCK = 128;
-
+// would pull every field of the state into local memory with it.  Measured
+// against it on the mid scene: its top staged in shared memory (extend 72.0 ->
+// 77.9 ms with 8 entries, 78.6 with 16: the per-access branch and the smaller
+// L1 cost more than the bank-parallel accesses save), and entries that carry
+// the child's entry distance, so that a pop can drop what lies beyond the best
+// hit (9 % fewer node visits, but every access twice as wide: extend 69.7 ->
+// 71.9 ms, on the heavy scene 28.9 -> 32.8).
 struct TraceStack {
-#if PT_SMEM_STACK
-    int* sm; // this thread's column of the block's shared array
-    int loc[STACK_SIZE - STACK_SMEM];
-    __device__ __forceinline__ TraceStack()
-    {
-        __shared__ int s_stack[STACK_SMEM * STACK_BLOCK];
-        sm = s_stack + threadIdx.x;
-    }
-    __device__ __forceinline__ int get(int i) const { return i < STACK_SMEM ? sm[i * STACK_BLOCK] : loc[i - STACK_SMEM]; }
-    __device__ __forceinline__ void set(int i, int v)
-    {
-        if (i < STACK_SMEM)
-            sm[i * STACK_BLOCK] = v;
-        else
-            loc[i - STACK_SMEM] = v;
-    }
-#else
     int loc[STACK_SIZE];
     __device__ __forceinline__ int get(int i) const { return loc[i]; }
     __device__ __forceinline__ void set(int i, int v) { loc[i] = v; }
-#endif
 };
 
 __device__ __forceinline__ void closest_begin(const DevScene& s, f3 o, f3 d, float tmin, float tmax, ClosestTrace& t, TraceStack& stack)
@@ -604,56 +610,65 @@ __device__ __forceinline__ void closest_begin(const DevScene& s, f3 o, f3 d, flo
     t.iter = 0;
 }
 
-template <bool W4>
-__device__ __forceinline__ bool closest_step(const DevScene& s, ClosestTrace& t, TraceStack& stack, TraceCounters& tc)
+// Ends a traversal at the next pop (the bottom of the stack is REF_DONE).
+__device__ __forceinline__ bool end_trace(int& sp)
 {
-    if (t.iter >= s.max_iterations) {
-        // A well-formed BVH never gets here; a malformed one must not hang the GPU.
-        atomicOr(s.error_word, ERR_WATCHDOG);
-        return true;
-    }
-    t.iter++;
-    const int ref = t.ref;
-    if (ref >= 0) {
-        PT_CHECK_INDEX((uint32_t)ref < s.node_count, s, return true)
-        tc.nodes++;
-        if (W4)
-            step4(s, t.r, t.tmin, t.h.t, t.ref, stack, t.sp);
-        else
-            step2(s, t.r, t.tmin, t.h.t, t.ref, stack, t.sp);
-        return false;
-    }
-    if (ref == REF_DONE)
-        return true;
-    if (ref == REF_EXIT_BLAS) {
+    sp = 1;
+    return true;
+}
+
+// Pops the next reference of a ray; leaving an instance restores the world
+// ray on the way.  True when the stack is exhausted.
+template <class Trace>
+__device__ __forceinline__ bool pop_ref(Trace& t, const TraceStack& stack)
+{
+    t.ref = stack.get(--t.sp);
+    if (t.ref == REF_EXIT_BLAS) { // never two in a row: instances are entered from the TLAS only
         t.r = t.world;
         t.in_blas = false;
         t.ref = stack.get(--t.sp);
-        return false;
     }
+    return t.ref == REF_DONE;
+}
+
+// The node step of closest_step (t.ref >= 0); true when the ray must pop.
+template <bool W4>
+__device__ __forceinline__ bool closest_node(const DevScene& s, ClosestTrace& t, TraceStack& stack, TraceCounters& tc)
+{
+    PT_CHECK_INDEX((uint32_t)t.ref < s.node_count, s, return end_trace(t.sp))
+    tc.nodes++;
+    return !(W4 ? step4<true>(s, t.r, t.tmin, t.h.t, t.ref, stack, t.sp) : step2(s, t.r, t.tmin, t.h.t, t.ref, stack, t.sp));
+}
+
+// The leaf step of closest_step (t.ref < 0), an instance entry or triangles;
+// true when the ray must pop.
+__device__ __forceinline__ bool closest_leaf(const DevScene& s, ClosestTrace& t, TraceStack& stack, TraceCounters& tc)
+{
+    const int ref = t.ref;
+    if (ref == REF_DONE) // an empty scene
+        return end_trace(t.sp);
+    if (ref == REF_EMPTY) // an unused slot of a 4-wide node, met by a NaN ray
+        return true;
     const uint32_t first = leaf_first(ref), count = leaf_count(ref);
     if (!t.in_blas) {
         // TLAS leaf: instances [first, first + count); one per leaf here.
-        PT_CHECK_INDEX(first < s.instance_count, s, return true)
+        PT_CHECK_INDEX(first < s.instance_count, s, return end_trace(t.sp))
         t.cur_inst = first;
         const DevInstance* di = s.dinst + first;
         const int root = __ldg(&di->blas_root);
-        if (root == REF_EMPTY || count != 1) {
-            t.ref = stack.get(--t.sp);
-            return false;
-        }
-        to_object(di, t.world.o, t.world.d, t.r);
+        if (root == REF_EMPTY || count != 1)
+            return true;
         if (t.sp >= STACK_SIZE) {
             atomicOr(s.error_word, ERR_STACK_OVERFLOW);
-            t.ref = stack.get(--t.sp);
-            return false;
+            return true;
         }
+        to_object(di, t.world.o, t.world.d, t.r);
         stack.set(t.sp++, REF_EXIT_BLAS);
         t.in_blas = true;
         t.ref = root;
         return false;
     }
-    PT_CHECK_INDEX((uint64_t)first + count <= s.tri_count, s, return true)
+    PT_CHECK_INDEX((uint64_t)first + count <= s.tri_count, s, return end_trace(t.sp))
     tc.tris += count;
     for (uint32_t k = 0; k < count; k++) {
         const TriRec* tr = s.tris + first + k;
@@ -670,8 +685,28 @@ __device__ __forceinline__ bool closest_step(const DevScene& s, ClosestTrace& t,
             t.found = true;
         }
     }
-    t.ref = stack.get(--t.sp);
+    return true;
+}
+
+// The watchdog of a traversal step: a well-formed BVH never gets there; a
+// malformed one must not hang the GPU.
+__device__ __forceinline__ bool out_of_steps(const DevScene& s, uint32_t& iter)
+{
+    if (iter >= s.max_iterations) {
+        atomicOr(s.error_word, ERR_WATCHDOG);
+        return true;
+    }
+    iter++;
     return false;
+}
+
+template <bool W4>
+__device__ __forceinline__ bool closest_step(const DevScene& s, ClosestTrace& t, TraceStack& stack, TraceCounters& tc)
+{
+    if (out_of_steps(s, t.iter))
+        return true;
+    const bool pop = t.ref >= 0 ? closest_node<W4>(s, t, stack, tc) : closest_leaf(s, t, stack, tc);
+    return pop && pop_ref(t, stack); // one copy of the pop: node and leaf lanes pop together
 }
 
 // A closest-hit traversal paused after a step budget (its "parking"): what a
@@ -907,42 +942,30 @@ __device__ __forceinline__ void shadow_begin(const DevScene& s, f3 o, f3 d, floa
 // Visibility of a finished shadow ray.
 __device__ __forceinline__ float shadow_result(const ShadowTrace& t) { return t.throughput < 1e-5f ? 0.0f : t.throughput; }
 
+// The node step of shadow_step (t.ref >= 0).
 template <bool W4>
-__device__ __forceinline__ bool shadow_step(const DevScene& s, ShadowTrace& t, TraceStack& stack, TraceCounters& tc)
+__device__ __forceinline__ bool shadow_node(const DevScene& s, ShadowTrace& t, TraceStack& stack, TraceCounters& tc)
 {
-    if (t.iter >= s.max_iterations) {
-        // A well-formed BVH never gets here; a malformed one must not hang the GPU.
-        atomicOr(s.error_word, ERR_WATCHDOG);
-        return true;
-    }
-    t.iter++;
+    PT_CHECK_INDEX((uint32_t)t.ref < s.node_count, s, return end_trace(t.sp))
+    tc.nodes++;
+    return !(W4 ? step4<false>(s, t.r, t.tmin, t.tmax, t.ref, stack, t.sp) : step2(s, t.r, t.tmin, t.tmax, t.ref, stack, t.sp));
+}
+
+// The leaf step of shadow_step (t.ref < 0): an instance entry or triangles.
+__device__ __forceinline__ bool shadow_leaf(const DevScene& s, ShadowTrace& t, TraceStack& stack, TraceCounters& tc)
+{
     const int ref = t.ref;
-    if (ref >= 0) {
-        PT_CHECK_INDEX((uint32_t)ref < s.node_count, s, return true)
-        tc.nodes++;
-        if (W4)
-            step4<false>(s, t.r, t.tmin, t.tmax, t.ref, stack, t.sp);
-        else
-            step2(s, t.r, t.tmin, t.tmax, t.ref, stack, t.sp);
-        return false;
-    }
-    if (ref == REF_DONE)
+    if (ref == REF_DONE) // an empty scene
+        return end_trace(t.sp);
+    if (ref == REF_EMPTY) // an unused slot of a 4-wide node, met by a NaN ray
         return true;
-    if (ref == REF_EXIT_BLAS) {
-        t.r = t.world;
-        t.in_blas = false;
-        t.ref = stack.get(--t.sp);
-        return false;
-    }
     const uint32_t first = leaf_first(ref), count = leaf_count(ref);
     if (!t.in_blas) {
-        PT_CHECK_INDEX(first < s.instance_count, s, return true)
+        PT_CHECK_INDEX(first < s.instance_count, s, return end_trace(t.sp))
         const DevInstance* di = s.dinst + first;
         const int root = __ldg(&di->blas_root);
-        if (root == REF_EMPTY || count != 1) {
-            t.ref = stack.get(--t.sp);
-            return false;
-        }
+        if (root == REF_EMPTY || count != 1)
+            return true;
         const uint32_t flags = __ldg(&di->flags);
         t.inst = first;
         t.opaque = (flags & 1u) != 0;
@@ -953,18 +976,17 @@ __device__ __forceinline__ bool shadow_step(const DevScene& s, ShadowTrace& t, T
             t.alpha_inst = first;
             t.alpha_pass = 1.0f - __ldg(&s.materials[mi].base_colour.w);
         }
-        to_object(di, t.world.o, t.world.d, t.r);
         if (t.sp >= STACK_SIZE) {
             atomicOr(s.error_word, ERR_STACK_OVERFLOW);
-            t.ref = stack.get(--t.sp);
-            return false;
+            return true;
         }
+        to_object(di, t.world.o, t.world.d, t.r);
         stack.set(t.sp++, REF_EXIT_BLAS);
         t.in_blas = true;
         t.ref = root;
         return false;
     }
-    PT_CHECK_INDEX((uint64_t)first + count <= s.tri_count, s, return true)
+    PT_CHECK_INDEX((uint64_t)first + count <= s.tri_count, s, return end_trace(t.sp))
     tc.tris += count;
     for (uint32_t k = 0; k < count; k++) {
         const TriRec* tr = s.tris + first + k;
@@ -984,10 +1006,60 @@ __device__ __forceinline__ bool shadow_step(const DevScene& s, ShadowTrace& t, T
                 break;
         }
     }
-    if (t.throughput == 0.0f || t.throughput < 1e-5f)
+    if (t.throughput < 1e-5f)
+        t.sp = 1; // occluded: the next pop ends the ray
+    return true;
+}
+
+template <bool W4>
+__device__ __forceinline__ bool shadow_step(const DevScene& s, ShadowTrace& t, TraceStack& stack, TraceCounters& tc)
+{
+    if (out_of_steps(s, t.iter))
         return true;
-    t.ref = stack.get(--t.sp);
-    return false;
+    const bool pop = t.ref >= 0 ? shadow_node<W4>(s, t, stack, tc) : shadow_leaf(s, t, stack, tc);
+    return pop && pop_ref(t, stack);
+}
+
+// One step of a whole warp's traversals: the lanes whose ray is at a node and
+// those at a leaf wait for one another, and the larger group steps.  Stepping
+// both groups in turn costs a warp the instructions of both on nearly every
+// iteration (a ray has about six node steps to each leaf step, so some lane is
+// nearly always at a leaf): on the mid scene at 1024 x 1024, 128 spp extend
+// went from 79.1 to 69.7 ms and on the heavy scene at 1920 x 1080, 4 spp from
+// 32.4 to 28.9; letting the leaves go at half or only at twice as many lanes
+// was 2-7 % slower.  Each
+// ray goes through the same steps as alone.  Called by all lanes of a warp
+// (`live`: the lane has an unfinished ray); true for a lane whose ray ends.
+__device__ __forceinline__ bool leaves_step(bool live, int ref)
+{
+    const unsigned nodes = __ballot_sync(0xffffffffu, live && ref >= 0), leaves = __ballot_sync(0xffffffffu, live && ref < 0);
+    return __popc(leaves) >= __popc(nodes);
+}
+
+template <bool W4>
+__device__ __forceinline__ bool closest_step_warp(const DevScene& s, bool live, ClosestTrace& t, TraceStack& stack, TraceCounters& tc)
+{
+    bool pop = false;
+    if (leaves_step(live, t.ref)) {
+        if (live && t.ref < 0)
+            pop = out_of_steps(s, t.iter) ? end_trace(t.sp) : closest_leaf(s, t, stack, tc);
+    } else if (live && t.ref >= 0) {
+        pop = out_of_steps(s, t.iter) ? end_trace(t.sp) : closest_node<W4>(s, t, stack, tc);
+    }
+    return pop && pop_ref(t, stack);
+}
+
+template <bool W4>
+__device__ __forceinline__ bool shadow_step_warp(const DevScene& s, bool live, ShadowTrace& t, TraceStack& stack, TraceCounters& tc)
+{
+    bool pop = false;
+    if (leaves_step(live, t.ref)) {
+        if (live && t.ref < 0)
+            pop = out_of_steps(s, t.iter) ? end_trace(t.sp) : shadow_leaf(s, t, stack, tc);
+    } else if (live && t.ref >= 0) {
+        pop = out_of_steps(s, t.iter) ? end_trace(t.sp) : shadow_node<W4>(s, t, stack, tc);
+    }
+    return pop && pop_ref(t, stack);
 }
 
 // Parking of an any-hit (shadow) traversal in the slots of TraceParking:

@@ -1,5 +1,6 @@
 // render_mega.cu — megakernel path tracer: one thread owns one pixel and runs
 // its samples back to back, tracing closest-hit and shadow rays inline.
+#define PT_NARROW_NODE_LOADS 1 // device/scene.cuh
 #include "device/render.cuh"
 #include "kernels.h"
 

@@ -244,9 +244,9 @@ enum Traversal : int { TRAV_BVH4 = 0, TRAV_BVH2 = 1, TRAV_BVH2_WW = 2 };
 // is deeper than PARK_STACK, or that finds no free slot, finishes here.  The
 // hit is the same either way: the resumed traversal continues the same
 // sequence of steps.
-// Residency: 8 blocks of 128 per SM (64 registers, 40-52 B of spills) over
-// the half-precision 4-wide nodes; 7 blocks measured 74.2 against 71.9 ms of
-// extend per step on the mid scene (the shadow kernel is faster at 7).
+// Residency: 8 blocks of 128 per SM (64 registers, 32-40 B of spills) over
+// the half-precision 4-wide nodes; on the heavy scene 7 blocks measured 25.2
+// against 24.5 ms of extend (on the mid scene 58.9 and 58.7).
 template <class Src, int TRAV, bool BUDGET = false>
 __global__ void __launch_bounds__(128, TRAV == TRAV_BVH4 ? 8 : 1) k_wf_extend(WaveArgs<Src> a, uint32_t qi, uint32_t budget)
 {
@@ -254,7 +254,6 @@ __global__ void __launch_bounds__(128, TRAV == TRAV_BVH4 ? 8 : 1) k_wf_extend(Wa
     const uint32_t count = *(volatile uint32_t*)&a.w.counts[qi];
     unsigned lane = threadIdx.x & 31;
     TraceCounters tc{0u, 0u};
-    uint32_t misses = 0;
     while (true) {
         uint32_t base = 0;
         if (lane == 0)
@@ -264,60 +263,57 @@ __global__ void __launch_bounds__(128, TRAV == TRAV_BVH4 ? 8 : 1) k_wf_extend(Wa
             break;
         uint32_t i = base + lane;
         uint32_t p = 0;
-        bool hit = false;
         bool ok = i < count;
         if (ok) {
             p = queue[i];
             PT_CHECK_ENTRY(ok, p, a)
         }
-        if (TRAV == TRAV_BVH4 && BUDGET) {
-            // one warp-uniform loop (a single copy of the step code): at
-            // iteration `budget` the lanes still traversing park together
-            ClosestTrace t;
-            TraceStack stack;
-            const uint32_t job = ok ? a.src.job_of(p) : 0u;
-            bool live = ok;
+        if (TRAV == TRAV_BVH2_WW) {
             if (ok) {
+                const DevScene& s = a.src.args(a.src.job_of(p)).s;
                 const float4 o = a.w.ray_o[p], d = a.w.ray_d[p];
-                closest_begin(a.src.args(job).s, mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), o.w, d.w, t, stack);
-            }
-            for (uint32_t k = 0;; k++) {
-                if (k == budget) {
-                    const bool park = live && t.sp <= PARK_STACK;
-                    const unsigned want = __ballot_sync(0xffffffffu, park);
-                    if (want) {
-                        uint32_t slot0 = 0;
-                        const int leader = __ffs(want) - 1;
-                        if ((int)lane == leader)
-                            slot0 = atomicAdd(&a.w.counts[6], (uint32_t)__popc(want));
-                        slot0 = __shfl_sync(0xffffffffu, slot0, leader);
-                        const uint32_t slot = slot0 + __popc(want & ((1u << lane) - 1u));
-                        if (park && slot < a.w.park.cap) {
-                            park_closest(a.w.park, slot, p, t, stack);
-                            live = false;
-                        }
-                    }
-                }
-                if (!__any_sync(0xffffffffu, live))
-                    break;
-                if (live && closest_step<true>(a.src.args(job).s, t, stack, tc)) {
-                    a.w.hit[p] = make_float4(t.h.t, t.h.b1, t.h.b2, __uint_as_float(t.h.inst));
-                    a.w.hit_prim[p] = t.found ? t.h.prim : 0xFFFFFFFFu;
-                    live = false;
-                }
+                Hit h;
+                const bool hit = trace_closest_ww(s, mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), o.w, d.w, h, tc);
+                a.w.hit[p] = make_float4(h.t, h.b1, h.b2, __uint_as_float(h.inst));
+                a.w.hit_prim[p] = hit ? h.prim : 0xFFFFFFFFu;
             }
             continue;
         }
-        if (!BUDGET && ok) {
-            const DevScene& s = a.src.args(a.src.job_of(p)).s;
-            float4 o = a.w.ray_o[p], d = a.w.ray_d[p];
-            Hit h;
-            if (TRAV == TRAV_BVH2_WW)
-                hit = trace_closest_ww(s, mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), o.w, d.w, h, tc);
-            else
-                hit = trace_closest_inl<TRAV == TRAV_BVH4>(s, mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), o.w, d.w, h, tc);
-            a.w.hit[p] = make_float4(h.t, h.b1, h.b2, __uint_as_float(h.inst));
-            a.w.hit_prim[p] = hit ? h.prim : 0xFFFFFFFFu;
+        // one warp-uniform loop (a single copy of the step code): with a step
+        // budget, the lanes still traversing at iteration `budget` park together
+        ClosestTrace t;
+        TraceStack stack;
+        t.ref = REF_DONE;
+        const DevScene& s = a.src.args(ok ? a.src.job_of(p) : 0u).s;
+        bool live = ok;
+        if (ok) {
+            const float4 o = a.w.ray_o[p], d = a.w.ray_d[p];
+            closest_begin(s, mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), o.w, d.w, t, stack);
+        }
+        for (uint32_t k = 0;; k++) {
+            if (BUDGET && k == budget) {
+                const bool park = live && t.sp <= PARK_STACK;
+                const unsigned want = __ballot_sync(0xffffffffu, park);
+                if (want) {
+                    uint32_t slot0 = 0;
+                    const int leader = __ffs(want) - 1;
+                    if ((int)lane == leader)
+                        slot0 = atomicAdd(&a.w.counts[6], (uint32_t)__popc(want));
+                    slot0 = __shfl_sync(0xffffffffu, slot0, leader);
+                    const uint32_t slot = slot0 + __popc(want & ((1u << lane) - 1u));
+                    if (park && slot < a.w.park.cap) {
+                        park_closest(a.w.park, slot, p, t, stack);
+                        live = false;
+                    }
+                }
+            }
+            if (!__any_sync(0xffffffffu, live))
+                break;
+            if (closest_step_warp<TRAV == TRAV_BVH4>(s, live, t, stack, tc)) {
+                a.w.hit[p] = make_float4(t.h.t, t.h.b1, t.h.b2, __uint_as_float(t.h.inst));
+                a.w.hit_prim[p] = t.found ? t.h.prim : 0xFFFFFFFFu;
+                live = false;
+            }
         }
     }
     uint32_t nodes = __reduce_add_sync(0xffffffffu, tc.nodes);
@@ -348,16 +344,20 @@ __global__ void __launch_bounds__(128, 8) k_wf_extend_resume(WaveArgs<Src> a)
         bool ok = slot < count;
         uint32_t p = ok ? a.w.park.path[slot] : 0u;
         PT_CHECK_ENTRY(ok, p, a)
+        ClosestTrace t;
+        TraceStack stack;
+        t.ref = REF_DONE;
+        const DevScene& s = a.src.args(ok ? a.src.job_of(p) : 0u).s;
         if (ok) {
-            const DevScene& s = a.src.args(a.src.job_of(p)).s;
             const float4 o = a.w.ray_o[p], d = a.w.ray_d[p];
-            ClosestTrace t;
-            TraceStack stack;
             resume_closest(s, a.w.park, slot, mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), o.w, t, stack);
-            while (!closest_step<true>(s, t, stack, tc)) {
+        }
+        while (__any_sync(0xffffffffu, ok)) {
+            if (closest_step_warp<true>(s, ok, t, stack, tc)) {
+                a.w.hit[p] = make_float4(t.h.t, t.h.b1, t.h.b2, __uint_as_float(t.h.inst));
+                a.w.hit_prim[p] = t.found ? t.h.prim : 0xFFFFFFFFu;
+                ok = false;
             }
-            a.w.hit[p] = make_float4(t.h.t, t.h.b1, t.h.b2, __uint_as_float(t.h.inst));
-            a.w.hit_prim[p] = t.found ? t.h.prim : 0xFFFFFFFFu;
         }
     }
     const uint32_t nodes = __reduce_add_sync(0xffffffffu, tc.nodes);
@@ -700,46 +700,38 @@ __global__ void __launch_bounds__(128, W4 ? 7 : 1) k_wf_shadow(WaveArgs<Src> a, 
         bool ok = i < count;
         uint32_t p = ok ? a.w.shadow_queue[i] : 0u;
         PT_CHECK_ENTRY(ok, p, a)
-        if (W4 && BUDGET) {
-            ShadowTrace t;
-            TraceStack stack;
-            const uint32_t job = ok ? a.src.job_of(p) : 0u;
-            bool live = ok;
-            if (ok) {
-                const float4 o = a.w.nee_o[p], d = a.w.nee_d[p];
-                shadow_begin(a.src.args(job).s, mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), 0.0f, o.w, t, stack);
-            }
-            for (uint32_t k = 0;; k++) {
-                if (k == budget) {
-                    const bool park = live && t.sp <= PARK_STACK;
-                    const unsigned want = __ballot_sync(0xffffffffu, park);
-                    if (want) {
-                        uint32_t slot0 = 0;
-                        const int leader = __ffs(want) - 1;
-                        if ((int)lane == leader)
-                            slot0 = atomicAdd(&a.w.counts[8], (uint32_t)__popc(want));
-                        slot0 = __shfl_sync(0xffffffffu, slot0, leader);
-                        const uint32_t slot = slot0 + __popc(want & ((1u << lane) - 1u));
-                        if (park && slot < a.w.park.cap) {
-                            park_shadow(a.w.park, slot, p, t, stack);
-                            live = false;
-                        }
+        ShadowTrace t;
+        TraceStack stack;
+        t.ref = REF_DONE;
+        const DevScene& s = a.src.args(ok ? a.src.job_of(p) : 0u).s;
+        bool live = ok;
+        if (ok) {
+            const float4 o = a.w.nee_o[p], d = a.w.nee_d[p];
+            shadow_begin(s, mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), 0.0f, o.w, t, stack);
+        }
+        for (uint32_t k = 0;; k++) {
+            if (BUDGET && k == budget) {
+                const bool park = live && t.sp <= PARK_STACK;
+                const unsigned want = __ballot_sync(0xffffffffu, park);
+                if (want) {
+                    uint32_t slot0 = 0;
+                    const int leader = __ffs(want) - 1;
+                    if ((int)lane == leader)
+                        slot0 = atomicAdd(&a.w.counts[8], (uint32_t)__popc(want));
+                    slot0 = __shfl_sync(0xffffffffu, slot0, leader);
+                    const uint32_t slot = slot0 + __popc(want & ((1u << lane) - 1u));
+                    if (park && slot < a.w.park.cap) {
+                        park_shadow(a.w.park, slot, p, t, stack);
+                        live = false;
                     }
                 }
-                if (!__any_sync(0xffffffffu, live))
-                    break;
-                if (live && shadow_step<true>(a.src.args(job).s, t, stack, tc)) {
-                    shadow_finish(a, p, shadow_result(t));
-                    live = false;
-                }
             }
-            continue;
-        }
-        if (ok) {
-            const DevScene& s = a.src.args(a.src.job_of(p)).s;
-            float4 o = a.w.nee_o[p], d = a.w.nee_d[p];
-            float vis = trace_shadow_inl<W4>(s, mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), 0.0f, o.w, tc);
-            shadow_finish(a, p, vis);
+            if (!__any_sync(0xffffffffu, live))
+                break;
+            if (shadow_step_warp<W4>(s, live, t, stack, tc)) {
+                shadow_finish(a, p, shadow_result(t));
+                live = false;
+            }
         }
     }
     uint32_t nodes = __reduce_add_sync(0xffffffffu, tc.nodes);
@@ -769,15 +761,19 @@ __global__ void __launch_bounds__(128, 7) k_wf_shadow_resume(WaveArgs<Src> a)
         bool ok = slot < count;
         uint32_t p = ok ? a.w.park.path[slot] : 0u;
         PT_CHECK_ENTRY(ok, p, a)
+        ShadowTrace t;
+        TraceStack stack;
+        t.ref = REF_DONE;
+        const DevScene& s = a.src.args(ok ? a.src.job_of(p) : 0u).s;
         if (ok) {
-            const DevScene& s = a.src.args(a.src.job_of(p)).s;
             const float4 o = a.w.nee_o[p], d = a.w.nee_d[p];
-            ShadowTrace t;
-            TraceStack stack;
             resume_shadow(s, a.w.park, slot, mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), 0.0f, o.w, t, stack);
-            while (!shadow_step<true>(s, t, stack, tc)) {
+        }
+        while (__any_sync(0xffffffffu, ok)) {
+            if (shadow_step_warp<true>(s, ok, t, stack, tc)) {
+                shadow_finish(a, p, shadow_result(t));
+                ok = false;
             }
-            shadow_finish(a, p, shadow_result(t));
         }
     }
     const uint32_t nodes = __reduce_add_sync(0xffffffffu, tc.nodes);
