@@ -1,7 +1,8 @@
 // render_wave.cu — wavefront path tracer.
 //
 // A wave renders `k` consecutive samples of every pixel: N = k * W * H paths.
-// Path state lives in structure-of-arrays buffers indexed by path id; stages
+// Path state lives in structure-of-arrays buffers indexed by path id (order.h:
+// neighbouring ids are samples of the same and neighbouring pixels); stages
 // exchange compact queues of path ids:
 //
 //   raygen      camera rays of all N paths (pathtrace.rg.hlsl:18-35)
@@ -31,6 +32,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "device/order.h"
 #include "device/render.cuh"
 #include "kernels.h"
 
@@ -38,7 +40,7 @@ namespace pt {
 
 // Pixel and sample of a path, and the job it belongs to.
 struct PathLoc {
-    uint32_t job, pix, si;
+    uint32_t job, px, py, si;
 };
 
 struct OneJob {
@@ -49,18 +51,23 @@ struct OneJob {
     uint32_t n_paths;      // k * W * H
     __device__ __forceinline__ PathLoc assign(uint32_t p) const
     {
-        uint32_t j = p / pixels;
-        return PathLoc{0u, p - j * pixels, first_sample + j};
+        uint32_t q, j;
+        path_place(p, pixels, samples, q, j);
+        PathLoc L;
+        L.job = 0u;
+        L.si = first_sample + j;
+        ordered_pixel(q, r.width, r.height, L.px, L.py);
+        return L;
     }
     __device__ __forceinline__ PathLoc locate(uint32_t p) const { return assign(p); }
     __device__ __forceinline__ uint32_t job_of(uint32_t) const { return 0u; }
     __device__ __forceinline__ const RenderArgs& args(uint32_t) const { return r; }
     __device__ __forceinline__ unsigned long long* counters() const { return r.counters; }
     __device__ __forceinline__ uint32_t accum_threads() const { return pixels; }
-    // the share (the whole wave) and the pixel of accumulation thread t
-    __device__ __forceinline__ const WaveShare share_of_pixel(uint32_t t, uint32_t& pix) const
+    // the share (the whole wave) of accumulation thread t and its place in the share's pixel order
+    __device__ __forceinline__ const WaveShare share_of_pixel(uint32_t t, uint32_t& q) const
     {
-        pix = t;
+        q = t;
         return WaveShare{0u, 0u, 0u, first_sample, samples, pixels};
     }
 };
@@ -76,9 +83,14 @@ struct ManyJobs {
     __device__ __forceinline__ PathLoc from_share(uint32_t e, uint32_t p) const
     {
         const WaveShare& E = shares[e];
-        uint32_t lp = p - E.path_base;
-        uint32_t j = lp / E.pixels;
-        return PathLoc{E.job, lp - j * E.pixels, E.first_sample + j};
+        const uint32_t lp = p - E.path_base;
+        uint32_t q, j;
+        path_place(lp, E.pixels, E.samples, q, j);
+        PathLoc L;
+        L.job = E.job;
+        L.si = E.first_sample + j;
+        ordered_pixel(q, jobs[E.job].width, jobs[E.job].height, L.px, L.py);
+        return L;
     }
     __device__ __forceinline__ PathLoc assign(uint32_t p) const
     {
@@ -98,7 +110,7 @@ struct ManyJobs {
     __device__ __forceinline__ const RenderArgs& args(uint32_t job) const { return jobs[job]; }
     __device__ __forceinline__ unsigned long long* counters() const { return ctr; }
     __device__ __forceinline__ uint32_t accum_threads() const { return n_pixels; }
-    __device__ __forceinline__ const WaveShare share_of_pixel(uint32_t t, uint32_t& pix) const
+    __device__ __forceinline__ const WaveShare share_of_pixel(uint32_t t, uint32_t& q) const
     {
         uint32_t lo = 0, hi = share_count;
         while (hi - lo > 1) {
@@ -109,7 +121,7 @@ struct ManyJobs {
                 hi = mid;
         }
         const WaveShare E = shares[lo];
-        pix = t - E.pixel_base;
+        q = t - E.pixel_base;
         return E;
     }
 };
@@ -186,10 +198,9 @@ __global__ void __launch_bounds__(256) k_wf_raygen(WaveArgs<Src> a)
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < a.src.n_paths; p += gridDim.x * blockDim.x) {
         const PathLoc L = a.src.assign(p);
         const RenderArgs& R = a.src.args(L.job);
-        uint32_t px = L.pix % R.width, py = L.pix / R.width;
-        uint32_t si = L.si;
+        const uint32_t px = L.px, py = L.py;
         Sampler smp;
-        sampler_start(smp, px, py, si, 0);
+        sampler_start(smp, px, py, L.si, 0);
         f2 u_pixel = sample_2d(smp);
         f2 u_lens = sample_2d(smp);
         f3 ro, rd;
@@ -473,15 +484,13 @@ __global__ void __launch_bounds__(128, MINB) k_wf_shade(WaveArgs<Src> a, uint32_
             const PathLoc L = a.src.locate(p);
             const RenderArgs& R = a.src.args(L.job);
             const DevScene& s = R.s;
-            uint32_t px = L.pix % R.width, py = L.pix / R.width;
-            uint32_t si = L.si;
             PathState pl;
             float4 t4 = a.w.tp[p], r4 = a.w.rad[p];
             pl.throughput = mk3(t4.x, t4.y, t4.z);
             pl.brdf_pdf = t4.w;
             pl.radiance = mk3(r4.x, r4.y, r4.z);
             pl.final_segment = sg >= R.max_bounces;
-            sampler_start(pl.smp, px, py, si, sg + 1);
+            sampler_start(pl.smp, L.px, L.py, L.si, sg + 1);
             float4 o = a.w.ray_o[p], d = a.w.ray_d[p];
             f3 ro = mk3(o.x, o.y, o.z), rd = mk3(d.x, d.y, d.z);
             uint32_t prim = a.w.hit_prim[p];
@@ -802,9 +811,11 @@ template <class Src>
 __global__ void __launch_bounds__(256) k_wf_accumulate(WaveArgs<Src> a)
 {
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < a.src.accum_threads(); t += gridDim.x * blockDim.x) {
-        uint32_t pix;
-        const WaveShare E = a.src.share_of_pixel(t, pix);
+        uint32_t q, px, py;
+        const WaveShare E = a.src.share_of_pixel(t, q);
         const RenderArgs& R = a.src.args(E.job);
+        ordered_pixel(q, R.width, R.height, px, py);
+        const uint32_t pix = py * R.width + px;
         float4 acc = R.image[pix];
         double s64[3] = {0.0, 0.0, 0.0};
         if (R.sum64) {
@@ -817,17 +828,16 @@ __global__ void __launch_bounds__(256) k_wf_accumulate(WaveArgs<Src> a)
             fa = feat_load(R.feat_a, pix, R.fp16_features);
             fn = feat_load(R.feat_n, pix, R.fp16_features);
             for (uint32_t j = 0; j < E.samples; j++) {
-                const size_t q = E.path_base + (size_t)j * E.pixels + pix;
-                feature_mean(fa, a.w.f_a[q], E.first_sample + j);
-                feature_mean(fn, a.w.f_n[q], E.first_sample + j);
+                const size_t path = E.path_base + path_at(q, j, E.pixels, E.samples);
+                feature_mean(fa, a.w.f_a[path], E.first_sample + j);
+                feature_mean(fn, a.w.f_n[path], E.first_sample + j);
             }
             feat_store(R.feat_a, pix, fa, R.fp16_features);
             feat_store(R.feat_n, pix, fn, R.fp16_features);
         }
         // FP64 sums only when the render keeps them: FP64 adds are slow on this GPU
         const bool want64 = R.sum64 != nullptr;
-        for (uint32_t j = 0; j < E.samples; j++) {
-            float4 r4 = a.w.rad[E.path_base + (size_t)j * E.pixels + pix];
+        auto add = [&](const float4& r4, uint32_t j) {
             f3 r = correct_radiance(mk3(r4.x, r4.y, r4.z) * R.exposure);
             accumulate(acc, r, E.first_sample + j);
             if (R.snapshot && E.first_sample + j + 1 == R.snapshot_after)
@@ -837,7 +847,23 @@ __global__ void __launch_bounds__(256) k_wf_accumulate(WaveArgs<Src> a)
                 s64[1] += (double)r.y;
                 s64[2] += (double)r.z;
             }
+        };
+        // a pixel's samples of a group are side by side (order.h): a group's
+        // reads are issued together
+        const float4* rad = a.w.rad + E.path_base;
+        uint32_t j = 0;
+        for (; j + SAMPLE_GROUP <= E.samples; j += SAMPLE_GROUP) {
+            const float4* g = rad + path_at(q, j, E.pixels, E.samples);
+            float4 v[SAMPLE_GROUP];
+#pragma unroll
+            for (uint32_t k = 0; k < SAMPLE_GROUP; k++)
+                v[k] = g[k];
+#pragma unroll
+            for (uint32_t k = 0; k < SAMPLE_GROUP; k++)
+                add(v[k], j + k);
         }
+        for (; j < E.samples; j++)
+            add(rad[path_at(q, j, E.pixels, E.samples)], j);
         R.image[pix] = acc;
         if (R.sum64) {
             double* d = R.sum64 + 4 * (size_t)pix;
