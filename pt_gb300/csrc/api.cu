@@ -325,6 +325,7 @@ void pt_destroy(pt_ctx* c)
             cudaEventDestroy(c->wave_join[k]);
         if (c->wave_acc[k])
             cudaEventDestroy(c->wave_acc[k]);
+        c->shadow_side[k].destroy();
     }
     if (c->wave_fork)
         cudaEventDestroy(c->wave_fork);
@@ -793,6 +794,12 @@ int pt_render(pt_ctx* c, const pt_render_params* p, pt_render_stats* stats)
             if (e != cudaSuccess)
                 return c->cuda_fail(e, "sub-wave stream");
         }
+        if (!timing) // stage timing records its events on one stream
+            for (int k = 0; k < ways; k++) {
+                cudaError_t e = c->shadow_side[k].create();
+                if (e != cudaSuccess)
+                    return c->cuda_fail(e, "shadow stream");
+            }
         if (ways > 1) {
             cudaError_t e = cudaSuccess;
             if (!c->wave_fork)
@@ -849,9 +856,11 @@ int pt_render(pt_ctx* c, const pt_render_params* p, pt_render_stats* stats)
             wm.stream[k] = k ? c->side[k] : c->stream;
             wm.join[k] = c->wave_join[k];
             wm.acc[k] = c->wave_acc[k];
+            if (!timing)
+                wm.shadow[k] = c->shadow_side[k];
         }
         cudaError_t e = launch_wavefront(a, c->wave_state.p, c->wave_state.n, n_paths, c->sm_count, &launches, c->stream,
-                                         timing ? &timer : nullptr, ways > 1 ? &wm : nullptr);
+                                         timing ? &timer : nullptr, wm);
         if (e != cudaSuccess)
             return c->cuda_fail(e, "wavefront launch");
         stage_marks = timer.count;

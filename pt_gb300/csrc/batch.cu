@@ -56,6 +56,7 @@ struct BatchState {
     uint32_t state2_paths = 0;
     cudaStream_t wave_side = nullptr;
     cudaEvent_t wfork = nullptr, wjoin = nullptr, wacc[2] = {nullptr, nullptr};
+    ShadowStream wshadow[2];
     bool w4 = true; // every job's scene has 4-wide nodes (else the BVH2 kernels run)
     DevBuf<unsigned long long> counters;
     DevBuf<uint32_t> error_word;
@@ -97,6 +98,8 @@ void batch_free(BatchState* b)
             cudaEventDestroy(e);
     for (cudaEvent_t e : b->done_ev)
         cudaEventDestroy(e);
+    for (ShadowStream& sh : b->wshadow)
+        sh.destroy();
     delete b;
 }
 
@@ -342,8 +345,11 @@ cudaError_t issue(pt_ctx* c, BatchState* b, const pt_batch_job* jobs, const std:
         uint32_t wl = 0;
         WaveMulti wm{};
         const bool two = plan.waves.size() >= 2 && b->state2_paths == b->state_paths;
+        wm.ways = 1;
+        wm.shadow[0] = b->wshadow[0];
         if (two) {
             wm.ways = 2;
+            wm.shadow[1] = b->wshadow[1];
             wm.state[1] = b->state2.p;
             wm.state_bytes[1] = b->state2.n;
             wm.stream[1] = b->wave_side;
@@ -354,7 +360,7 @@ cudaError_t issue(pt_ctx* c, BatchState* b, const pt_batch_job* jobs, const std:
         }
         e = launch_wavefront_batch(b->jobs.p, b->shares.p, plan.waves.data(), (uint32_t)plan.waves.size(), b->path_share.p,
                                    b->counters.p, b->state.p, b->state.n, b->state_paths, b->w4, c->sm_count, &wl, st,
-                                   two ? &wm : nullptr, two ? b->path_share2.p : nullptr, b->done_ev.data());
+                                   wm, two ? b->path_share2.p : nullptr, b->done_ev.data());
         if (e != cudaSuccess)
             return e;
         nl += wl;
@@ -522,6 +528,9 @@ int pt_render_batch(pt_ctx* c, const pt_batch_job* jobs, uint32_t count, uint32_
         for (cudaEvent_t* ev : {&b->ev0, &b->ev1})
             if (e == cudaSuccess)
                 e = cudaEventCreate(ev);
+        for (ShadowStream& sh : b->wshadow)
+            if (e == cudaSuccess)
+                e = sh.create();
         if (e == cudaSuccess)
             e = b->counters.alloc(8);
         if (e == cudaSuccess)

@@ -100,6 +100,7 @@ struct pt_ctx {
     uint32_t wave_paths_x[pt::MAX_WAVE_WAYS] = {};
     cudaStream_t side[pt::MAX_WAVE_WAYS] = {};
     cudaEvent_t wave_fork = nullptr, wave_join[pt::MAX_WAVE_WAYS] = {}, wave_acc[pt::MAX_WAVE_WAYS] = {};
+    pt::ShadowStream shadow_side[pt::MAX_WAVE_WAYS]; // one per sub-wave
     uint32_t wave_paths = 0;    // paths the wave state holds
     int sm_count = 0;
     pt_render_params camera{};  // pt_set_camera state

@@ -50,16 +50,27 @@ size_t wave_state_bytes(uint32_t n_paths_max);
 // snapshot exactly those of one stream.  fork / join[] tie the extra streams
 // to the launch's stream before and after.
 constexpr int MAX_WAVE_WAYS = 4;
+// The stream on which a wave's shadow rays are traced beside the next
+// segment's closest hits, and the events between the two: `shaded` after the
+// shade stage that queued them, `traced` after the shadow stage.
+struct ShadowStream {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t shaded = nullptr, traced = nullptr;
+    cudaError_t create();
+    void destroy();
+};
+
 struct WaveMulti {
     int ways;
     void* state[MAX_WAVE_WAYS];
     size_t state_bytes[MAX_WAVE_WAYS];
     cudaStream_t stream[MAX_WAVE_WAYS];
     cudaEvent_t fork, join[MAX_WAVE_WAYS], acc[MAX_WAVE_WAYS];
+    ShadowStream shadow[MAX_WAVE_WAYS]; // stream null: the stages of a wave run one after the other
 };
 cudaError_t launch_wavefront(const RenderArgs& r, void* state, size_t state_bytes, uint32_t n_paths_max, int sm_count,
-                             uint32_t* launches, cudaStream_t stream, StageTimer* timer = nullptr,
-                             const WaveMulti* multi = nullptr);
+                             uint32_t* launches, cudaStream_t stream, StageTimer* timer,
+                             const WaveMulti& multi);
 cudaError_t wave_init_tables(const uint32_t* table128, const float* srgb256, cudaStream_t stream);
 
 // Batched wavefront: waves hold shares of several jobs (RenderArgs in device
@@ -87,7 +98,7 @@ cudaError_t wave_batch_prepare();
 cudaError_t launch_wavefront_batch(const RenderArgs* jobs, const WaveShare* shares, const BatchWave* waves, uint32_t wave_count,
                                    uint32_t* path_share, unsigned long long* counters, void* state, size_t state_bytes,
                                    uint32_t n_paths_max, bool w4, int sm_count, uint32_t* launches, cudaStream_t stream,
-                                   const WaveMulti* multi = nullptr, uint32_t* path_share2 = nullptr,
+                                   const WaveMulti& multi, uint32_t* path_share2 = nullptr,
                                    cudaEvent_t* wave_done = nullptr);
 // Records `ev` on `st` so that its time can be read later: inside a stream
 // capture as an external event (an event-record node of the graph; a plain
