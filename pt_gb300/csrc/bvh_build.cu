@@ -24,10 +24,16 @@
 // has the smallest surface area (ties broken by the lower index pair, so the
 // globally closest pair in each segment is always mutual), mutual nearest
 // neighbours merge into a new node, and the survivors are compacted in
-// order, until each segment is one cluster.  Nodes are numbered in merge
-// order by prefix sums (deterministic).  PT_BVH=lbvh selects the radix tree
-// instead (kept for A/B).
+// order, until each segment is one cluster.  Rounds over all segments at once
+// run until every segment is small; then one block per segment finishes it in
+// shared memory.  Nodes are numbered in merge order by prefix sums
+// (deterministic).  PT_BVH=lbvh selects the radix tree instead (kept for A/B).
 #include <cub/cub.cuh>
+#include <thrust/iterator/counting_iterator.h>
+#include <thrust/iterator/transform_iterator.h>
+
+#include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 
@@ -100,12 +106,12 @@ struct Scratch {
     float4* c_hi[2];
     uint32_t* c_seg[2];
     int* nn;
-    uint32_t* m_flag;
-    uint32_t* a_flag;
-    uint32_t* m_scan;
-    uint32_t* a_scan;
-    uint32_t* counters; // [0] nodes emitted, [1] live clusters, [2] merges in the last round,
-                        // [3] 1 once a round merged nothing, [4] buffer holding the clusters
+    uint64_t* scan;     // exclusive sums of (merge flag << 32 | survivor flag)
+    uint32_t* counters; // rounds alternate between two pairs: [2p] nodes emitted, [2p + 1] live clusters at the
+                        // start of rounds of parity p; [4] the most live clusters of a segment, [5] segments that
+                        // have any
+    uint32_t* seg_live; // live clusters of each segment when its block takes over,
+    uint32_t* seg_first; // and the first of them
     void* scan_temp;
     size_t scan_bytes;
     // leaf collapse of the BLAS trees
@@ -135,10 +141,36 @@ size_t cub_sort_bytes(uint32_t n)
     return bytes;
 }
 
+// Merge and survivor flags of cluster i, (merge << 32) | survivor: mutual
+// nearest neighbours merge and the lower index of a pair keeps the merged
+// cluster; zero past the live count.
+struct PlocFlags {
+    const int* nn;
+    const uint32_t* live;
+    __host__ __device__ uint64_t operator()(int i) const
+    {
+#ifdef __CUDA_ARCH__
+        if (i >= (int)*live)
+            return 0;
+        const int j = nn[i];
+        const bool mutual = j >= 0 && nn[j] == i;
+        return (mutual && i < j ? 1ull << 32 : 0ull) | (mutual && i > j ? 0ull : 1ull);
+#else
+        return 0;
+#endif
+    }
+};
+using PlocFlagIter = thrust::transform_iterator<PlocFlags, thrust::counting_iterator<int>, uint64_t>;
+
+PlocFlagIter ploc_flags(const int* nn, const uint32_t* live)
+{
+    return PlocFlagIter(thrust::counting_iterator<int>(0), PlocFlags{nn, live});
+}
+
 size_t cub_scan_bytes(uint32_t n)
 {
     size_t bytes = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, bytes, (uint32_t*)nullptr, (uint32_t*)nullptr, (int)n);
+    cub::DeviceScan::ExclusiveSum(nullptr, bytes, ploc_flags(nullptr, nullptr), (uint64_t*)nullptr, (int)n);
     return bytes;
 }
 
@@ -172,10 +204,9 @@ Scratch carve_scratch(void* base, uint32_t n, uint32_t nseg)
         s.c_seg[b] = carve<uint32_t>(p, nn);
     }
     s.nn = carve<int>(p, nn);
-    s.m_flag = carve<uint32_t>(p, nn);
-    s.a_flag = carve<uint32_t>(p, nn);
-    s.m_scan = carve<uint32_t>(p, nn);
-    s.a_scan = carve<uint32_t>(p, nn);
+    s.scan = carve<uint64_t>(p, nn);
+    s.seg_live = carve<uint32_t>(p, nseg + 1);
+    s.seg_first = carve<uint32_t>(p, nseg + 1);
     s.counters = carve<uint32_t>(p, 8);
     s.cnt = carve<uint32_t>(p, nn);
     s.sah = carve<float>(p, nn);
@@ -221,43 +252,90 @@ __device__ __forceinline__ void atomic_bounds(int* b, float4 lo, float4 hi)
     atomicMax(b + 5, f2ord(hi.z));
 }
 
-__global__ void k_tri_boxes(BvhBuildInput in, Scratch s)
+// Bounds of the centroids (cb) and boxes (box, may be null) of a block's
+// primitives, all threads of the block calling.  When they are of one segment,
+// one thread's atomics for the whole block: with a thread each, 12 atomics per
+// triangle queued on a few addresses, and k_tri_boxes took 6,300 us for two
+// million triangles in 64 meshes, 33 us with this.
+constexpr int BOUNDS_THREADS = 256;
+
+__device__ __forceinline__ void segment_bounds(bool valid, uint32_t m, int* cb, int* box, float4 cen, float4 lo, float4 hi)
 {
-    uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= in.tri_count)
+    __shared__ int s_b[12][BOUNDS_THREADS / 32];
+    __shared__ uint32_t s_m;
+    if (threadIdx.x == 0) // valid in every block that is launched
+        s_m = m;
+    __syncthreads();
+    if (!__syncthreads_and(!valid || m == s_m)) {
+        if (valid) {
+            atomic_bounds(cb + 6 * m, cen, cen);
+            if (box)
+                atomic_bounds(box + 6 * m, lo, hi);
+        }
         return;
-    uint32_t m = upper_segment(in.mesh_tri_base, in.mesh_count, g);
-    uint32_t local = g - in.mesh_tri_base[m];
-    uint32_t ib = in.mesh_index_offset[m] + 3 * local;
-    uint32_t vb = in.mesh_vertex_offset[m];
-    float4 a = in.vertices[2 * (size_t)(vb + in.indices[ib + 0])];
-    float4 b = in.vertices[2 * (size_t)(vb + in.indices[ib + 1])];
-    float4 c = in.vertices[2 * (size_t)(vb + in.indices[ib + 2])];
-    float4 lo = make_float4(fminf(fminf(a.x, b.x), c.x), fminf(fminf(a.y, b.y), c.y), fminf(fminf(a.z, b.z), c.z), 0.0f);
-    float4 hi = make_float4(fmaxf(fmaxf(a.x, b.x), c.x), fmaxf(fmaxf(a.y, b.y), c.y), fmaxf(fmaxf(a.z, b.z), c.z), 0.0f);
-    s.lo[g] = lo;
-    s.hi[g] = hi;
-    s.seg[g] = m;
+    }
+    const int none_lo = 0x7FFFFFFF, none_hi = (int)0x80000000;
+    const int v[12] = {valid ? f2ord(cen.x) : none_lo, valid ? f2ord(cen.y) : none_lo, valid ? f2ord(cen.z) : none_lo,
+                       valid ? f2ord(cen.x) : none_hi, valid ? f2ord(cen.y) : none_hi, valid ? f2ord(cen.z) : none_hi,
+                       valid ? f2ord(lo.x) : none_lo,  valid ? f2ord(lo.y) : none_lo,  valid ? f2ord(lo.z) : none_lo,
+                       valid ? f2ord(hi.x) : none_hi,  valid ? f2ord(hi.y) : none_hi,  valid ? f2ord(hi.z) : none_hi};
+    const int warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < 12; k++) {
+        const int w = k % 6 < 3 ? __reduce_min_sync(0xffffffffu, v[k]) : __reduce_max_sync(0xffffffffu, v[k]);
+        if ((threadIdx.x & 31) == 0)
+            s_b[k][warp] = w;
+    }
+    __syncthreads();
+    if (threadIdx.x < (box ? 12 : 6)) {
+        const int k = threadIdx.x;
+        int w = s_b[k][0];
+        for (int i = 1; i < (int)(blockDim.x / 32); i++)
+            w = k % 6 < 3 ? min(w, s_b[k][i]) : max(w, s_b[k][i]);
+        int* to = (k < 6 ? cb : box) + 6 * s_m + k % 6;
+        if (k % 6 < 3)
+            atomicMin(to, w);
+        else
+            atomicMax(to, w);
+    }
+}
+
+__global__ void __launch_bounds__(BOUNDS_THREADS) k_tri_boxes(BvhBuildInput in, Scratch s)
+{
+    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool valid = g < in.tri_count;
+    uint32_t m = 0;
+    float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
+    if (valid) {
+        m = upper_segment(in.mesh_tri_base, in.mesh_count, g);
+        uint32_t local = g - in.mesh_tri_base[m];
+        uint32_t ib = in.mesh_index_offset[m] + 3 * local;
+        uint32_t vb = in.mesh_vertex_offset[m];
+        float4 a = in.vertices[2 * (size_t)(vb + in.indices[ib + 0])];
+        float4 b = in.vertices[2 * (size_t)(vb + in.indices[ib + 1])];
+        float4 c = in.vertices[2 * (size_t)(vb + in.indices[ib + 2])];
+        lo = make_float4(fminf(fminf(a.x, b.x), c.x), fminf(fminf(a.y, b.y), c.y), fminf(fminf(a.z, b.z), c.z), 0.0f);
+        hi = make_float4(fmaxf(fmaxf(a.x, b.x), c.x), fmaxf(fmaxf(a.y, b.y), c.y), fmaxf(fmaxf(a.z, b.z), c.z), 0.0f);
+        s.lo[g] = lo;
+        s.hi[g] = hi;
+        s.seg[g] = m;
+    }
     float4 cen = make_float4(0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z), 0.0f);
-    atomic_bounds(s.seg_cb + 6 * m, cen, cen);
-    atomic_bounds(s.seg_box + 6 * m, lo, hi);
+    segment_bounds(valid, m, s.seg_cb, s.seg_box, cen, lo, hi);
 }
 
 // World box of each instance: the 8 corners of its mesh box under the
 // object-to-world transform, padded.
-__global__ void k_inst_boxes(BvhBuildInput in, const int* mesh_box, Scratch s)
+__device__ __forceinline__ void instance_box(const BvhBuildInput& in, const int* mesh_box, uint32_t i, float4& lo, float4& hi)
 {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= in.instance_count)
-        return;
     uint32_t m = in.inst_mesh[i];
     const int* mb = mesh_box + 6 * m;
     float blo[3] = {ord2f(mb[0]), ord2f(mb[1]), ord2f(mb[2])};
     float bhi[3] = {ord2f(mb[3]), ord2f(mb[4]), ord2f(mb[5])};
     const DevInstanceData& d = in.inst_data[i];
     float4 rows[3] = {d.t0, d.t1, d.t2};
-    float4 lo = make_float4(__int_as_float(0x7f800000), __int_as_float(0x7f800000), __int_as_float(0x7f800000), 0.0f);
-    float4 hi = make_float4(-lo.x, -lo.y, -lo.z, 0.0f);
+    lo = make_float4(__int_as_float(0x7f800000), __int_as_float(0x7f800000), __int_as_float(0x7f800000), 0.0f);
+    hi = make_float4(-lo.x, -lo.y, -lo.z, 0.0f);
     if (!(blo[0] <= bhi[0])) {
         // empty mesh: a point at the instance origin (its BLAS root is empty)
         lo = make_float4(rows[0].w, rows[1].w, rows[2].w, 0.0f);
@@ -276,11 +354,21 @@ __global__ void k_inst_boxes(BvhBuildInput in, const int* mesh_box, Scratch s)
             hi.z = fmaxf(hi.z, w[2]);
         }
     }
-    s.lo[i] = lo;
-    s.hi[i] = hi;
-    s.seg[i] = 0;
+}
+
+__global__ void __launch_bounds__(BOUNDS_THREADS) k_inst_boxes(BvhBuildInput in, const int* mesh_box, Scratch s)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool valid = i < in.instance_count;
+    float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
+    if (valid) {
+        instance_box(in, mesh_box, i, lo, hi);
+        s.lo[i] = lo;
+        s.hi[i] = hi;
+        s.seg[i] = 0;
+    }
     float4 cen = make_float4(0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z), 0.0f);
-    atomic_bounds(s.seg_cb, cen, cen);
+    segment_bounds(valid, 0, s.seg_cb, nullptr, cen, lo, hi);
 }
 
 __global__ void k_morton(Scratch s, uint32_t n)
@@ -496,111 +584,348 @@ __global__ void k_ploc_init(Scratch s, uint32_t n, int mode_tlas)
     s.c_seg[0][pos] = (uint32_t)(s.keys_out[pos] >> KEY_SEG_SHIFT);
 }
 
-// (min, max) index pair order for ties between equal distances
-__device__ __forceinline__ bool pair_before(int i, int j, int k)
+// Nearest neighbours of clusters `own` and own + 1 (own even) among the
+// clusters k0 .. k1 + 1 (k0, k1 even) staged in shared memory, `stride` floats
+// each of lo.x, lo.y, lo.z, hi.x, hi.y, hi.z: of those at most `radius` away (and
+// of the own segment, SEG; below n otherwise) the one whose box merges with the
+// smallest surface, of equal ones the first (the lower index pair).  Two boxes
+// are read at a time, four distances per six 8-byte reads.
+template <bool SEG>
+__device__ __forceinline__ void nn_pair(const float* box, int stride, const uint32_t* seg, int own, int k0, int k1, int n, int radius,
+                                        int& j0, int& j1)
 {
-    const int a0 = min(i, j), a1 = max(i, j), b0 = min(i, k), b1 = max(i, k);
-    return a0 < b0 || (a0 == b0 && a1 < b1);
-}
-
-// The round kernels read the live cluster count (counters[1]) and whether
-// the rounds are over (counters[3]) from device memory, so rounds run back to
-// back without the host; grids and scans cover `cap` >= live positions.
-__global__ void k_ploc_nn(const float4* lo, const float4* hi, const uint32_t* seg, const uint32_t* counters, int radius, int* nn)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int n = (int)counters[1];
-    if (counters[3] || i >= n)
-        return;
-    const float4 li = lo[i], hi_i = hi[i];
-    const uint32_t si = seg[i];
-    float best = 0.0f;
-    int bj = -1;
-    const int j0 = max(0, i - radius), j1 = min(n - 1, i + radius);
-    for (int j = j0; j <= j1; j++) {
-        if (j == i || seg[j] != si)
-            continue;
-        const float d = half_area(box_min(li, lo[j]), box_max(hi_i, hi[j]));
-        if (bj < 0 || d < best || (d == best && pair_before(i, j, bj))) {
-            best = d;
-            bj = j;
-        }
+    auto pair_at = [&](int row, int k) { return *reinterpret_cast<const float2*>(box + row * stride + k); };
+    const float2 ax = pair_at(0, own), ay = pair_at(1, own), az = pair_at(2, own);
+    const float2 bx = pair_at(3, own), by = pair_at(4, own), bz = pair_at(5, own);
+    uint2 as = make_uint2(0u, 0u);
+    if (SEG)
+        as = *reinterpret_cast<const uint2*>(seg + own);
+    float best0 = 0.0f, best1 = 0.0f;
+    j0 = j1 = -1;
+#pragma unroll (SEG ? 4 : 1) // the block kernel has no registers to spare
+    for (int k = k0; k <= k1; k += 2) {
+        const float2 cx = pair_at(0, k), cy = pair_at(1, k), cz = pair_at(2, k);
+        const float2 dx = pair_at(3, k), dy = pair_at(4, k), dz = pair_at(5, k);
+        uint2 cs = make_uint2(0u, k + 1 < n ? 0u : 1u);
+        if (SEG)
+            cs = *reinterpret_cast<const uint2*>(seg + k);
+        // half the surface of the merged box of own + q and k + r, and whether it is the best so far
+#define PT_NN_TRY(q, r, i, j, best, jbest)                                                                     \
+    {                                                                                                          \
+        const float ex = fmaxf(bx.q, dx.r) - fminf(ax.q, cx.r), ey = fmaxf(by.q, dy.r) - fminf(ay.q, cy.r),    \
+                    ez = fmaxf(bz.q, dz.r) - fminf(az.q, cz.r);                                                \
+        const float d = ex * ey + ey * ez + ez * ex;                                                           \
+        const int off = (j) - (i);                                                                             \
+        if (cs.r == as.q && off != 0 && off >= -radius && off <= radius && (jbest < 0 || d < best)) {          \
+            best = d;                                                                                          \
+            jbest = (j);                                                                                       \
+        }                                                                                                      \
     }
-    nn[i] = bj;
-}
-
-// Mutual nearest neighbours merge; the lower index of a pair keeps the merged
-// cluster.  Positions past the live count get zero flags (the scans cover cap).
-__global__ void k_ploc_flags(const int* nn, const uint32_t* counters, int cap, uint32_t* m_flag, uint32_t* a_flag)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= cap || counters[3])
-        return;
-    if (i >= (int)counters[1]) {
-        m_flag[i] = 0u;
-        a_flag[i] = 0u;
-        return;
+        PT_NN_TRY(x, x, own, k, best0, j0)
+        PT_NN_TRY(x, y, own, k + 1, best0, j0)
+        PT_NN_TRY(y, x, own + 1, k, best1, j1)
+        PT_NN_TRY(y, y, own + 1, k + 1, best1, j1)
+#undef PT_NN_TRY
     }
-    const int j = nn[i];
-    const bool mutual = j >= 0 && nn[j] == i;
-    m_flag[i] = (mutual && i < j) ? 1u : 0u;
-    a_flag[i] = (mutual && i > j) ? 0u : 1u;
 }
 
-__global__ void k_ploc_merge(Scratch s, int cur, BvhNode* nodes, int node_base)
+// Nearest neighbours of all live clusters: a block stages its NN_CLUSTERS
+// clusters and the window on either side.  Bound by the arithmetic of the
+// n (2 radius + 1) distances: two million clusters 230 us (381 with a thread
+// to a cluster reading the boxes through L1), 10,000 10 us (29).
+constexpr int NN_THREADS = 128, NN_CLUSTERS = 2 * NN_THREADS;
+
+__global__ void __launch_bounds__(NN_THREADS) k_ploc_nn(const float4* lo, const float4* hi, const uint32_t* seg, const uint32_t* live,
+                                                        int radius, int* nn)
+{
+    extern __shared__ __align__(16) float s_box[]; // lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, segment: `span` of each
+    const int n = (int)*live;
+    const int base = blockIdx.x * NN_CLUSTERS;
+    if (base >= n)
+        return;
+    const int pad = (radius + 1) & ~1, span = NN_CLUSTERS + 2 * pad;
+    uint32_t* s_seg = reinterpret_cast<uint32_t*>(s_box + 6 * span);
+    for (int k = threadIdx.x; k < span; k += NN_THREADS) {
+        const int j = base - pad + k;
+        const bool in = j >= 0 && j < n;
+        const float4 a = in ? lo[j] : make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = in ? hi[j] : a;
+        s_box[k] = a.x;
+        s_box[span + k] = a.y;
+        s_box[2 * span + k] = a.z;
+        s_box[3 * span + k] = b.x;
+        s_box[4 * span + k] = b.y;
+        s_box[5 * span + k] = b.z;
+        s_seg[k] = in ? seg[j] : 0xFFFFFFFFu; // no segment has this number
+    }
+    __syncthreads();
+    const int i0 = base + 2 * threadIdx.x;
+    if (i0 >= n)
+        return;
+    const int own = pad + 2 * threadIdx.x;
+    int j0, j1;
+    nn_pair<true>(s_box, span, s_seg, own, own - pad, own + pad, span, radius, j0, j1);
+    nn[i0] = j0 < 0 ? -1 : base - pad + j0;
+    if (i0 + 1 < n)
+        nn[i0 + 1] = j1 < 0 ? -1 : base - pad + j1;
+}
+
+__device__ __forceinline__ BvhNode merged_node(float4 lo0, float4 hi0, int ref0, float4 lo1, float4 hi1, int ref1)
+{
+    float4 blo[2], bhi[2];
+    padded(lo0, hi0, blo[0], bhi[0]);
+    padded(lo1, hi1, blo[1], bhi[1]);
+    BvhNode nd;
+    nd.c0xy = make_float4(blo[0].x, bhi[0].x, blo[0].y, bhi[0].y);
+    nd.c1xy = make_float4(blo[1].x, bhi[1].x, blo[1].y, bhi[1].y);
+    nd.c01z = make_float4(blo[0].z, bhi[0].z, blo[1].z, bhi[1].z);
+    nd.link = make_int4(ref0, ref1, 0, 0);
+    return nd;
+}
+
+// Merges the pairs of round `parity` and compacts the survivors into the other
+// cluster buffer; the last cluster's thread writes the next round's counters.
+__global__ void k_ploc_merge(Scratch s, int parity, BvhNode* nodes, int node_base)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s.counters[3] || i >= (int)s.counters[1] || !s.a_flag[i])
+    const int n = (int)s.counters[2 * parity + 1];
+    if (i >= n)
         return;
-    const int nxt = cur ^ 1;
-    const uint32_t o = s.a_scan[i];
-    const float4 lo = s.c_lo[cur][i], hi = s.c_hi[cur][i];
-    if (s.m_flag[i]) {
+    const uint64_t flags = PlocFlags{s.nn, &s.counters[2 * parity + 1]}(i);
+    const uint64_t before = s.scan[i];
+    const uint32_t nodes_before = s.counters[2 * parity];
+    const int nxt = parity ^ 1;
+    if (i == n - 1) {
+        const uint64_t total = before + flags;
+        s.counters[2 * nxt] = nodes_before + (uint32_t)(total >> 32);
+        s.counters[2 * nxt + 1] = (uint32_t)total;
+    }
+    if (!(uint32_t)flags)
+        return;
+    const uint32_t o = (uint32_t)before;
+    float4 lo = s.c_lo[parity][i], hi = s.c_hi[parity][i];
+    int ref = s.c_ref[parity][i];
+    if (flags >> 32) {
         const int j = s.nn[i];
-        const float4 lo_j = s.c_lo[cur][j], hi_j = s.c_hi[cur][j];
-        const int node = (int)(s.counters[0] + s.m_scan[i]);
-        float4 blo[2], bhi[2];
-        padded(lo, hi, blo[0], bhi[0]);
-        padded(lo_j, hi_j, blo[1], bhi[1]);
-        BvhNode nd;
-        nd.c0xy = make_float4(blo[0].x, bhi[0].x, blo[0].y, bhi[0].y);
-        nd.c1xy = make_float4(blo[1].x, bhi[1].x, blo[1].y, bhi[1].y);
-        nd.c01z = make_float4(blo[0].z, bhi[0].z, blo[1].z, bhi[1].z);
-        nd.link = make_int4(s.c_ref[cur][i], s.c_ref[cur][j], 0, 0);
-        nodes[node_base + node] = nd;
-        s.c_ref[nxt][o] = node_base + node;
-        s.c_lo[nxt][o] = box_min(lo, lo_j);
-        s.c_hi[nxt][o] = box_max(hi, hi_j);
-    } else {
-        s.c_ref[nxt][o] = s.c_ref[cur][i];
-        s.c_lo[nxt][o] = lo;
-        s.c_hi[nxt][o] = hi;
+        const float4 lo_j = s.c_lo[parity][j], hi_j = s.c_hi[parity][j];
+        const int node = node_base + (int)(nodes_before + (uint32_t)(before >> 32));
+        nodes[node] = merged_node(lo, hi, ref, lo_j, hi_j, s.c_ref[parity][j]);
+        ref = node;
+        lo = box_min(lo, lo_j);
+        hi = box_max(hi, hi_j);
     }
-    s.c_seg[nxt][o] = s.c_seg[cur][i];
+    s.c_ref[nxt][o] = ref;
+    s.c_lo[nxt][o] = lo;
+    s.c_hi[nxt][o] = hi;
+    s.c_seg[nxt][o] = s.c_seg[parity][i];
 }
 
-// End of a round: the clusters now sit in buffer `nxt`; a round without a
-// merge ends the rounds (every non-empty segment is one cluster).
-__global__ void k_ploc_count(Scratch s, int nxt)
+// First live cluster and live count of each segment (clusters keep their
+// segments' order), and the most of any.
+__global__ void k_ploc_segments(Scratch s, int parity, uint32_t nseg)
 {
-    if (s.counters[3])
+    const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= nseg)
         return;
-    const int n = (int)s.counters[1];
-    const uint32_t merges = s.m_scan[n - 1] + s.m_flag[n - 1];
-    s.counters[0] += merges;
-    s.counters[1] = s.a_scan[n - 1] + s.a_flag[n - 1];
-    s.counters[2] = merges;
-    s.counters[4] = (uint32_t)nxt;
-    if (merges == 0 || s.counters[1] <= 1)
-        s.counters[3] = 1u;
+    const uint32_t n = s.counters[2 * parity + 1];
+    const uint32_t* seg = s.c_seg[parity];
+    auto first_at_least = [&](uint32_t v) {
+        uint32_t a = 0, b = n;
+        while (a < b) {
+            const uint32_t mid = (a + b) >> 1;
+            if (seg[mid] < v)
+                a = mid + 1;
+            else
+                b = mid;
+        }
+        return a;
+    };
+    const uint32_t first = first_at_least(m), live = first_at_least(m + 1) - first;
+    s.seg_first[m] = first;
+    s.seg_live[m] = live;
+    atomicMax(&s.counters[4], live);
+    if (live)
+        atomicAdd(&s.counters[5], 1u);
 }
 
-__global__ void k_ploc_roots(Scratch s)
+// Finishes the segments with lo_count < live clusters <= CAP, one block each:
+// the same rounds as above on the segment's clusters in shared memory.  A
+// segment's merges do not depend on the others', so the tree is the one that
+// rounds over all segments would give (only the nodes' numbers differ).  The
+// rounds' launches and scans, at 25 us a round however few clusters were left,
+// took most of the build: 36,000 triangles in 56 meshes and 232 instances 3.2
+// ms, 0.87 ms with this; two million in 64 meshes and 10,256 instances 13.4 and
+// 3.1 ms with the search and bounds above.  While fewer clusters than threads are left, several
+// lanes share a cluster's window.
+template <int THREADS, int CAP>
+__global__ void __launch_bounds__(THREADS) k_ploc_block(Scratch s, int parity, BvhNode* nodes, int node_base, uint32_t lo_count, int radius)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int cur = (int)s.counters[4];
-    if (i < (int)s.counters[1])
-        s.seg_root[s.c_seg[cur][i]] = s.c_ref[cur][i];
+    constexpr int PER = CAP / THREADS;
+    extern __shared__ __align__(16) float s_box[]; // CAP each of lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, reference, neighbour
+    int* s_ref = reinterpret_cast<int*>(s_box + 6 * CAP);
+    int* s_nn = s_ref + CAP;
+    __shared__ uint32_t s_warp[THREADS / 32], s_total, s_rank;
+    const uint32_t m = blockIdx.x;
+    uint32_t n = s.seg_live[m];
+    if (n == 0 || n <= lo_count || n > (uint32_t)CAP)
+        return;
+    const uint32_t first = s.seg_first[m], tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (n == 1) {
+        if (tid == 0)
+            s.seg_root[m] = s.c_ref[parity][first];
+        return;
+    }
+    // this segment's nodes come after those of the segments before it: one per cluster less one per segment
+    if (tid == 0)
+        s_rank = 0;
+    __syncthreads();
+    uint32_t filled = 0;
+    for (uint32_t k = tid; k < m; k += THREADS)
+        filled += s.seg_live[k] != 0 ? 1u : 0u;
+    if (filled)
+        atomicAdd(&s_rank, filled);
+    for (uint32_t k = tid; k < n; k += THREADS) {
+        const float4 a = s.c_lo[parity][first + k], b = s.c_hi[parity][first + k];
+        s_box[k] = a.x;
+        s_box[CAP + k] = a.y;
+        s_box[2 * CAP + k] = a.z;
+        s_box[3 * CAP + k] = b.x;
+        s_box[4 * CAP + k] = b.y;
+        s_box[5 * CAP + k] = b.z;
+        s_ref[k] = s.c_ref[parity][first + k];
+    }
+    __syncthreads();
+    int node = node_base + (int)(s.counters[2 * parity] + first - s_rank);
+    auto box_lo = [&](int k) { return make_float4(s_box[k], s_box[CAP + k], s_box[2 * CAP + k], 0.0f); };
+    auto box_hi = [&](int k) { return make_float4(s_box[3 * CAP + k], s_box[4 * CAP + k], s_box[5 * CAP + k], 0.0f); };
+    while (n > 1) { // every round merges at least one pair
+        if (n > THREADS) {
+            const int pad = (radius + 1) & ~1;
+            for (int own = 2 * (int)tid; own < (int)n; own += 2 * THREADS) {
+                int j0, j1;
+                nn_pair<false>(s_box, CAP, nullptr, own, max(0, own - pad), min(own + pad, ((int)n - 1) & ~1), (int)n, radius, j0, j1);
+                s_nn[own] = j0;
+                if (own + 1 < (int)n)
+                    s_nn[own + 1] = j1;
+            }
+        }
+        // lanes per cluster: as many as the block has to spare (a power of two)
+        uint32_t share = 1;
+        while (share < 32 && 2 * share * n <= THREADS)
+            share *= 2;
+        for (uint32_t k = tid; n <= THREADS && k < (n * share + 31) / 32 * 32; k += THREADS) { // whole warps: the shuffles below
+            const int i = (int)(k / share), sub = (int)(k % share);
+            float best = 0.0f;
+            int bj = -1;
+            if (i < (int)n) {
+                const float4 li = box_lo(i), hi_i = box_hi(i);
+                const int j_end = min((int)n - 1, i + radius);
+#pragma unroll 4
+                for (int j = max(0, i - radius) + sub; j <= j_end; j += (int)share) {
+                    const float d = half_area(box_min(li, box_lo(j)), box_max(hi_i, box_hi(j)));
+                    if (j != i && (bj < 0 || d < best)) {
+                        best = d;
+                        bj = j;
+                    }
+                }
+            }
+            for (uint32_t o = 1; o < share; o <<= 1) {
+                const float od = __shfl_xor_sync(0xffffffffu, best, o);
+                const int oj = __shfl_xor_sync(0xffffffffu, bj, o);
+                if (oj >= 0 && (bj < 0 || od < best || (od == best && oj < bj))) {
+                    best = od;
+                    bj = oj;
+                }
+            }
+            if (sub == 0 && i < (int)n)
+                s_nn[i] = bj;
+        }
+        __syncthreads();
+        // each thread's own run of clusters
+        const uint32_t per = (n + THREADS - 1) / THREADS;
+        uint32_t flags = 0, mine = 0; // flags: 2 bits each (survives, merges); mine: merges << 16 | survivors
+#pragma unroll
+        for (int c = 0; c < PER; c++) {
+            const int i = (int)(tid * per) + c;
+            if (c >= (int)per || i >= (int)n)
+                continue;
+            const int j = s_nn[i];
+            const bool mutual = s_nn[j] == i;
+            if (mutual && i > j)
+                continue;
+            flags |= (mutual ? 3u : 1u) << (2 * c);
+            mine += mutual ? (1u << 16) + 1u : 1u;
+        }
+        // exclusive sums over the block
+        uint32_t sum = mine;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= (uint32_t)o)
+                sum += v;
+        }
+        if (lane == 31)
+            s_warp[warp] = sum;
+        __syncthreads();
+        if (warp == 0) {
+            const uint32_t v = lane < THREADS / 32 ? s_warp[lane] : 0u;
+            uint32_t w = v;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xffffffffu, w, o);
+                if (lane >= (uint32_t)o)
+                    w += u;
+            }
+            if (lane < THREADS / 32)
+                s_warp[lane] = w - v;
+            if (lane == 31)
+                s_total = w;
+        }
+        __syncthreads();
+        // the survivors are read before any is overwritten
+        const uint32_t before = s_warp[warp] + sum - mine;
+        float4 lo[PER], hi[PER];
+        int ref[PER];
+        int id = node + (int)(before >> 16);
+#pragma unroll
+        for (int c = 0; c < PER; c++) {
+            const uint32_t fl = (flags >> (2 * c)) & 3u;
+            if (!fl)
+                continue;
+            const int i = (int)(tid * per) + c;
+            lo[c] = box_lo(i);
+            hi[c] = box_hi(i);
+            ref[c] = s_ref[i];
+            if (fl & 2u) {
+                const int j = s_nn[i];
+                const float4 lo_j = box_lo(j), hi_j = box_hi(j);
+                nodes[id] = merged_node(lo[c], hi[c], ref[c], lo_j, hi_j, s_ref[j]);
+                lo[c] = box_min(lo[c], lo_j);
+                hi[c] = box_max(hi[c], hi_j);
+                ref[c] = id++;
+            }
+        }
+        __syncthreads();
+        int o = (int)(before & 0xFFFFu);
+#pragma unroll
+        for (int c = 0; c < PER; c++) {
+            if (!((flags >> (2 * c)) & 3u))
+                continue;
+            s_box[o] = lo[c].x;
+            s_box[CAP + o] = lo[c].y;
+            s_box[2 * CAP + o] = lo[c].z;
+            s_box[3 * CAP + o] = hi[c].x;
+            s_box[4 * CAP + o] = hi[c].y;
+            s_box[5 * CAP + o] = hi[c].z;
+            s_ref[o] = ref[c];
+            o++;
+        }
+        const uint32_t total = s_total;
+        node += (int)(total >> 16);
+        n = total & 0xFFFFu;
+        __syncthreads();
+        if ((total >> 16) == 0)
+            break; // only boxes that are not numbers get here: the root is then any of the clusters
+    }
+    if (tid == 0)
+        s.seg_root[m] = s_ref[0];
 }
 
 // ---- SAH leaf collapse of the BLAS trees (PLOC output, leaves of one triangle)
@@ -816,50 +1141,69 @@ bool use_ploc_tlas()
     return v;
 }
 
-// PLOC rounds over the sorted primitives; they end when a round merges
-// nothing (then every non-empty segment is one cluster).  The rounds run in
-// chunks of PLOC_CHUNK back to back on the device (a round after the end does
-// nothing); the host reads the counters once per chunk, not once per round.
-constexpr uint32_t PLOC_CHUNK = 8;
+// PLOC over the sorted primitives: rounds over all segments until the largest
+// has at most PLOC_BLOCK_CAP clusters, then a block per segment.  A round takes
+// about 0.84 of the clusters to the next (0.56 the first), so the host
+// estimates how many are needed and looks at the counters once or twice.
+constexpr uint32_t PLOC_SMALL_CAP = 512, PLOC_BLOCK_CAP = 4096;
 
-cudaError_t build_ploc(Scratch& s, uint32_t n, BvhNode* nodes, int node_base, int mode_tlas, cudaStream_t st)
+template <int THREADS, int CAP>
+cudaError_t launch_ploc_block(const Scratch& s, int parity, uint32_t nseg, BvhNode* nodes, int node_base, uint32_t lo_count, int radius,
+                              cudaStream_t st)
 {
+    const int bytes = 8 * CAP * (int)sizeof(float);
+    cudaError_t e = cudaFuncSetAttribute(k_ploc_block<THREADS, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess)
+        return e;
+    k_ploc_block<THREADS, CAP><<<nseg, THREADS, bytes, st>>>(s, parity, nodes, node_base, lo_count, radius);
+    return cudaGetLastError();
+}
+
+cudaError_t build_ploc(Scratch& s, uint32_t n, uint32_t nseg, BvhNode* nodes, int node_base, int mode_tlas, cudaStream_t st)
+{
+    const int radius = ploc_radius(mode_tlas);
     k_ploc_init<<<blocks(n, 256), 256, 0, st>>>(s, n, mode_tlas);
-    cudaMemsetAsync(s.counters, 0, 8 * sizeof(uint32_t), st);
-    const uint32_t init[4] = {0u, n, 0u, n <= 1 ? 1u : 0u};
+    const uint32_t init[4] = {0u, n, 0u, 0u};
     cudaError_t e = cudaMemcpyAsync(s.counters, init, sizeof(init), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess)
         return e;
-    int cur = 0;
-    uint32_t cap = n, rounds = 0;
-    uint32_t c[5] = {0u, n, 0u, n <= 1 ? 1u : 0u, 0u};
-    while (!c[3]) {
-        if (rounds > n + PLOC_CHUNK)
-            return cudaErrorUnknown; // every round merges at least one pair while a segment has two clusters
-        for (uint32_t k = 0; k < PLOC_CHUNK; k++, rounds++) {
-            k_ploc_nn<<<blocks(cap, 128), 128, 0, st>>>(s.c_lo[cur], s.c_hi[cur], s.c_seg[cur], s.counters,
-                                                          ploc_radius(mode_tlas), s.nn);
-            k_ploc_flags<<<blocks(cap, 256), 256, 0, st>>>(s.nn, s.counters, (int)cap, s.m_flag, s.a_flag);
-            size_t bytes = s.scan_bytes;
-            e = cub::DeviceScan::ExclusiveSum(s.scan_temp, bytes, s.m_flag, s.m_scan, (int)cap, st);
-            if (e == cudaSuccess)
-                e = cub::DeviceScan::ExclusiveSum(s.scan_temp, bytes, s.a_flag, s.a_scan, (int)cap, st);
-            if (e != cudaSuccess)
-                return e;
-            k_ploc_merge<<<blocks(cap, 128), 128, 0, st>>>(s, cur, nodes, node_base);
-            k_ploc_count<<<1, 1, 0, st>>>(s, cur ^ 1);
-            cur ^= 1;
-        }
-        e = cudaMemcpyAsync(c, s.counters, 5 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+    const size_t nn_bytes = 7 * sizeof(float) * (size_t)(NN_CLUSTERS + 2 * ((radius + 1) & ~1));
+    int parity = 0;
+    uint32_t cap = n, rounds = 0, most = 0;
+    for (;;) {
+        if ((e = cudaMemsetAsync(&s.counters[4], 0, 2 * sizeof(uint32_t), st)) != cudaSuccess)
+            return e;
+        k_ploc_segments<<<blocks(nseg, 128), 128, 0, st>>>(s, parity, nseg);
+        uint32_t c[6];
+        e = cudaMemcpyAsync(c, s.counters, sizeof(c), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess)
             e = cudaStreamSynchronize(st);
         if (e != cudaSuccess)
             return e;
-        cap = c[1];
+        cap = c[2 * parity + 1];
+        most = c[4];
+        s.blas_nodes = n - c[5]; // a segment of k primitives gets k - 1 nodes
+        if (most <= PLOC_BLOCK_CAP)
+            break;
+        if (rounds > n)
+            return cudaErrorUnknown; // every round merges at least one pair while a segment has two clusters
+        const double ratio = (double)most / PLOC_BLOCK_CAP;
+        const uint32_t more = (uint32_t)std::ceil(std::log(rounds == 0 ? std::max(0.56 * ratio, 1.01) : ratio) / 0.174) + (rounds == 0 ? 1u : 0u);
+        for (uint32_t k = 0; k < std::min(std::max(more, 1u), 32u); k++, rounds++) {
+            const uint32_t* live = &s.counters[2 * parity + 1];
+            k_ploc_nn<<<blocks(cap, NN_CLUSTERS), NN_THREADS, nn_bytes, st>>>(s.c_lo[parity], s.c_hi[parity], s.c_seg[parity], live, radius,
+                                                                           s.nn);
+            size_t bytes = s.scan_bytes;
+            if ((e = cub::DeviceScan::ExclusiveSum(s.scan_temp, bytes, ploc_flags(s.nn, live), s.scan, (int)cap, st)) != cudaSuccess)
+                return e;
+            k_ploc_merge<<<blocks(cap, 128), 128, 0, st>>>(s, parity, nodes, node_base);
+            parity ^= 1;
+        }
     }
-    s.blas_nodes = c[0];
-    k_ploc_roots<<<blocks(c[1], 128), 128, 0, st>>>(s);
-    return cudaGetLastError();
+    e = launch_ploc_block<PLOC_SMALL_CAP / 2, PLOC_SMALL_CAP>(s, parity, nseg, nodes, node_base, 0u, radius, st);
+    if (e == cudaSuccess && most > PLOC_SMALL_CAP)
+        e = launch_ploc_block<1024, PLOC_BLOCK_CAP>(s, parity, nseg, nodes, node_base, PLOC_SMALL_CAP, radius, st);
+    return e;
 }
 
 float env_float(const char* name, float dflt)
@@ -911,7 +1255,7 @@ cudaError_t build_tree(Scratch& s, uint32_t n, uint32_t nseg, BvhNode* nodes, in
         return e;
     if (mode_tlas ? use_ploc_tlas() : use_ploc()) {
         k_small_roots<<<blocks(nseg, 128), 128, 0, st>>>(s, nseg, mode_tlas);
-        return build_ploc(s, n, nodes, node_base, mode_tlas, st);
+        return build_ploc(s, n, nseg, nodes, node_base, mode_tlas, st);
     }
     cudaMemsetAsync(s.parent, 0xFF, sizeof(int) * n, st);
     if (n > 1)
@@ -1048,7 +1392,7 @@ cudaError_t bvh_build(const BvhBuildInput& in, BvhBuildOutput& out, void* scratc
         if (in.tri_count > 0) {
             Scratch sb = s;
             sb.seg_box = mesh_box;
-            k_tri_boxes<<<blocks(in.tri_count, 256), 256, 0, st>>>(in, sb);
+            k_tri_boxes<<<blocks(in.tri_count, BOUNDS_THREADS), BOUNDS_THREADS, 0, st>>>(in, sb);
         }
         s.blas_nodes = 0;
         e = build_tree(s, in.tri_count, in.mesh_count, out.nodes, 0, 0, st);
