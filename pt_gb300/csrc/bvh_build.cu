@@ -324,48 +324,109 @@ __global__ void __launch_bounds__(BOUNDS_THREADS) k_tri_boxes(BvhBuildInput in, 
     segment_bounds(valid, m, s.seg_cb, s.seg_box, cen, lo, hi);
 }
 
-// World box of each instance: the 8 corners of its mesh box under the
-// object-to-world transform, padded.
-__device__ __forceinline__ void instance_box(const BvhBuildInput& in, const int* mesh_box, uint32_t i, float4& lo, float4& hi)
+// World boxes of the instances, one warp each: the box around the transformed
+// boxes of the mesh's tree eight levels down (up to 256), cut to the box of the
+// mesh box's eight transformed corners.  A rotated mesh fills little of the
+// latter (a sphere a third of its surface), and every ray that meets it enters
+// the instance.  Each lane follows the five bits of its number down the tree
+// and then takes the eight boxes three levels below.  Heavy scene (10,000
+// rotated grids and spheres) at 1920 x 1080, 4 spp: extend 22.3 -> 21.1 ms, shadow
+// 12.4 -> 11.6; mid scene (196 rotated boxes) at 1024 x 1024, 128 spp: 51.9 -> 50.7
+// and 24.0 -> 22.2.
+constexpr int BOX_LANE_LEVELS = 5, BOX_MORE_LEVELS = 3;
+
+// Box of node `ref`'s child on side `bit`, and the child.
+__device__ __forceinline__ int child_box(const BvhNode* nodes, int ref, uint32_t bit, float4& lo, float4& hi)
 {
-    uint32_t m = in.inst_mesh[i];
-    const int* mb = mesh_box + 6 * m;
-    float blo[3] = {ord2f(mb[0]), ord2f(mb[1]), ord2f(mb[2])};
-    float bhi[3] = {ord2f(mb[3]), ord2f(mb[4]), ord2f(mb[5])};
-    const DevInstanceData& d = in.inst_data[i];
-    float4 rows[3] = {d.t0, d.t1, d.t2};
-    lo = make_float4(__int_as_float(0x7f800000), __int_as_float(0x7f800000), __int_as_float(0x7f800000), 0.0f);
-    hi = make_float4(-lo.x, -lo.y, -lo.z, 0.0f);
-    if (!(blo[0] <= bhi[0])) {
-        // empty mesh: a point at the instance origin (its BLAS root is empty)
-        lo = make_float4(rows[0].w, rows[1].w, rows[2].w, 0.0f);
-        hi = lo;
-    } else {
-        for (int corner = 0; corner < 8; corner++) {
-            double p[3] = {(corner & 1) ? bhi[0] : blo[0], (corner & 2) ? bhi[1] : blo[1], (corner & 4) ? bhi[2] : blo[2]};
-            float w[3];
-            for (int r = 0; r < 3; r++)
-                w[r] = (float)((double)rows[r].x * p[0] + (double)rows[r].y * p[1] + (double)rows[r].z * p[2] + (double)rows[r].w);
-            lo.x = fminf(lo.x, w[0]);
-            lo.y = fminf(lo.y, w[1]);
-            lo.z = fminf(lo.z, w[2]);
-            hi.x = fmaxf(hi.x, w[0]);
-            hi.y = fmaxf(hi.y, w[1]);
-            hi.z = fmaxf(hi.z, w[2]);
-        }
-    }
+    const BvhNode nd = nodes[ref];
+    const float4 xy = bit ? nd.c1xy : nd.c0xy;
+    lo = make_float4(xy.x, xy.z, bit ? nd.c01z.z : nd.c01z.x, 0.0f);
+    hi = make_float4(xy.y, xy.w, bit ? nd.c01z.w : nd.c01z.y, 0.0f);
+    return bit ? nd.link.y : nd.link.x;
 }
 
-__global__ void __launch_bounds__(BOUNDS_THREADS) k_inst_boxes(BvhBuildInput in, const int* mesh_box, Scratch s)
+// Bounds of row . p + row.w over a box of centre c and half size h, widened by
+// `err` for the rounding of the single-precision sums.
+__device__ __forceinline__ void widen_by_row(float4 row, float4 c, float4 h, float err, float& lo, float& hi)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = i < in.instance_count;
+    const float mid = ((row.x * c.x + row.y * c.y) + row.z * c.z) + row.w;
+    const float ext = ((fabsf(row.x) * h.x + fabsf(row.y) * h.y) + fabsf(row.z) * h.z) + err;
+    lo = fminf(lo, mid - ext);
+    hi = fmaxf(hi, mid + ext);
+}
+
+__global__ void __launch_bounds__(BOUNDS_THREADS) k_inst_boxes(BvhBuildInput in, const int* mesh_box, const int* mesh_root,
+                                                               const BvhNode* nodes, Scratch s)
+{
+    const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    const bool valid = i < in.instance_count && lane == 0;
+    const float inf = __int_as_float(0x7f800000);
     float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
-    if (valid) {
-        instance_box(in, mesh_box, i, lo, hi);
-        s.lo[i] = lo;
-        s.hi[i] = hi;
-        s.seg[i] = 0;
+    if (i < in.instance_count) { // the whole warp
+        const uint32_t m = in.inst_mesh[i];
+        const int* mb = mesh_box + 6 * m;
+        const float blo[3] = {ord2f(mb[0]), ord2f(mb[1]), ord2f(mb[2])};
+        const float bhi[3] = {ord2f(mb[3]), ord2f(mb[4]), ord2f(mb[5])};
+        const DevInstanceData& d = in.inst_data[i];
+        const float4 rows[3] = {d.t0, d.t1, d.t2};
+        if (!(blo[0] <= bhi[0])) {
+            // empty mesh: a point at the instance origin (its BLAS root is empty)
+            lo = make_float4(rows[0].w, rows[1].w, rows[2].w, 0.0f);
+            hi = lo;
+        } else {
+            float clo[3], chi[3], tlo[3] = {inf, inf, inf}, thi[3] = {-inf, -inf, -inf}, err[3];
+            const double p[3] = {(lane & 1) ? bhi[0] : blo[0], (lane & 2) ? bhi[1] : blo[1], (lane & 4) ? bhi[2] : blo[2]};
+            const float mag[3] = {fmaxf(fabsf(blo[0]), fabsf(bhi[0])), fmaxf(fabsf(blo[1]), fabsf(bhi[1])),
+                                  fmaxf(fabsf(blo[2]), fabsf(bhi[2]))};
+#pragma unroll
+            for (int r = 0; r < 3; r++) {
+                clo[r] = chi[r] =
+                    (float)((double)rows[r].x * p[0] + (double)rows[r].y * p[1] + (double)rows[r].z * p[2] + (double)rows[r].w);
+                // at most 8 roundings of terms no larger than this sum (boxes are padded by 1e-5)
+                err[r] = 8.0f * 0x1p-24f * 1.001f *
+                         (((fabsf(rows[r].x) * mag[0] + fabsf(rows[r].y) * mag[1]) + fabsf(rows[r].z) * mag[2]) + fabsf(rows[r].w));
+            }
+            auto add = [&](float4 a, float4 b) {
+                const float4 c = make_float4(0.5f * (a.x + b.x), 0.5f * (a.y + b.y), 0.5f * (a.z + b.z), 0.0f);
+                const float4 h = make_float4(0.5f * (b.x - a.x), 0.5f * (b.y - a.y), 0.5f * (b.z - a.z), 0.0f);
+#pragma unroll
+                for (int r = 0; r < 3; r++)
+                    widen_by_row(rows[r], c, h, err[r], tlo[r], thi[r]);
+            };
+            int ref = mesh_root[m];
+            const bool single = ref < 0; // one leaf: no tree to follow
+            float4 a, b;
+            for (int l = 0; l < BOX_LANE_LEVELS && ref >= 0; l++)
+                ref = child_box(nodes, ref, (lane >> l) & 1u, a, b);
+            if (!single && ref < 0)
+                add(a, b);
+            for (uint32_t k = 0; ref >= 0 && k < (1u << BOX_MORE_LEVELS); k++) {
+                int c = ref;
+                for (int l = 0; l < BOX_MORE_LEVELS && c >= 0; l++)
+                    c = child_box(nodes, c, (k >> l) & 1u, a, b);
+                add(a, b);
+            }
+            float out[6];
+#pragma unroll
+            for (int r = 0; r < 3; r++) {
+                const float c0 = ord2f(__reduce_min_sync(0xffffffffu, f2ord(clo[r]))), c1 = ord2f(__reduce_max_sync(0xffffffffu, f2ord(chi[r])));
+                const float t0 = ord2f(__reduce_min_sync(0xffffffffu, f2ord(tlo[r]))), t1 = ord2f(__reduce_max_sync(0xffffffffu, f2ord(thi[r])));
+                const bool use = !single && t0 <= t1; // false for sums that are not numbers
+                out[r] = use ? fmaxf(c0, t0) : c0;
+                out[3 + r] = use ? fminf(c1, t1) : c1;
+                if (!(out[r] <= out[3 + r])) { // rounding pushed the two apart
+                    out[r] = c0;
+                    out[3 + r] = c1;
+                }
+            }
+            lo = make_float4(out[0], out[1], out[2], 0.0f);
+            hi = make_float4(out[3], out[4], out[5], 0.0f);
+        }
+        if (lane == 0) {
+            s.lo[i] = lo;
+            s.hi[i] = hi;
+            s.seg[i] = 0;
+        }
     }
     float4 cen = make_float4(0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z), 0.0f);
     segment_bounds(valid, 0, s.seg_cb, nullptr, cen, lo, hi);
@@ -1415,7 +1476,7 @@ cudaError_t bvh_build(const BvhBuildInput& in, BvhBuildOutput& out, void* scratc
     uint32_t tb[2] = {0, in.instance_count};
     k_init_bounds<<<1, 32, 0, st>>>(s.seg_cb, s.seg_box, s.seg_root, 1);
     cudaMemcpyAsync(s.seg_base, tb, sizeof(tb), cudaMemcpyHostToDevice, st);
-    k_inst_boxes<<<blocks(in.instance_count, 128), 128, 0, st>>>(in, mesh_box, s);
+    k_inst_boxes<<<blocks((uint64_t)in.instance_count * 32, BOUNDS_THREADS), BOUNDS_THREADS, 0, st>>>(in, mesh_box, out.mesh_root, out.nodes, s);
     e = build_tree(s, in.instance_count, 1, out.nodes, tlas_base, 1, st);
     if (e != cudaSuccess)
         return e;
