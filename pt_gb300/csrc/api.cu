@@ -484,6 +484,12 @@ int pt_upload_scene(pt_ctx* c, const pt_scene_view* v)
     c->instance_count = v->instance_count;
     c->material_count = v->material_count;
     c->has_ior = v->material_ior != nullptr && v->material_count != 0;
+    c->plain = !c->has_ior;
+    for (uint32_t i = 0; i < v->material_count && c->plain; i++) {
+        uint32_t bits;
+        std::memcpy(&bits, &v->materials[i].rough_metal_normal_map_bits[3], sizeof(bits));
+        c->plain = (bits & PT_ANY_MAP_BITS) == 0;
+    }
     c->texture_count = v->texture_count;
     c->light_words = v->light_word_count;
     c->light_count = v->light_count;
@@ -644,6 +650,7 @@ RenderArgs render_args(const pt_ctx* c, const pt_render_params* p, bool fp64)
     a.s.tlas_root = c->tlas_root;
     a.s.env = mk3(c->env[0], c->env[1], c->env[2]);
     a.s.error_word = c->error_word.p;
+    a.s.plain = c->plain ? 1u : 0u;
     std::memcpy(a.inv_view, p->inv_view, sizeof(a.inv_view));
     std::memcpy(a.inv_proj, p->inv_proj, sizeof(a.inv_proj));
     a.near_plane = p->near_plane;

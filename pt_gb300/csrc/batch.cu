@@ -58,6 +58,7 @@ struct BatchState {
     cudaEvent_t wfork = nullptr, wjoin = nullptr, wacc[2] = {nullptr, nullptr};
     ShadowStream wshadow[2];
     bool w4 = true; // every job's scene has 4-wide nodes (else the BVH2 kernels run)
+    bool plain = true; // no job's scene has maps or refraction
     DevBuf<unsigned long long> counters;
     DevBuf<uint32_t> error_word;
     cudaStream_t side = nullptr;
@@ -241,9 +242,11 @@ int prepare(pt_ctx* c, BatchState* b, const pt_batch_job* jobs, const std::vecto
     b->graph_key.clear();
     std::vector<RenderArgs> args(p.size());
     b->w4 = true;
+    b->plain = true;
     for (size_t j = 0; j < p.size(); j++) {
         RenderArgs a = render_args(jobs[j].scene, &p[j], false);
         b->w4 = b->w4 && a.s.nodes4 != nullptr;
+        b->plain = b->plain && a.s.plain != 0;
         a.image = b->image.p + b->img_off[j];
         a.sum64 = b->sum_off[j] == SIZE_MAX ? nullptr : b->sum64.p + 4 * b->sum_off[j];
         a.counters = b->counters.p;
@@ -359,7 +362,7 @@ cudaError_t issue(pt_ctx* c, BatchState* b, const pt_batch_job* jobs, const std:
             wm.acc[1] = b->wacc[1];
         }
         e = launch_wavefront_batch(b->jobs.p, b->shares.p, plan.waves.data(), (uint32_t)plan.waves.size(), b->path_share.p,
-                                   b->counters.p, b->state.p, b->state.n, b->state_paths, b->w4, c->sm_count, &wl, st,
+                                   b->counters.p, b->state.p, b->state.n, b->state_paths, b->w4, b->plain, c->sm_count, &wl, st,
                                    wm, two ? b->path_share2.p : nullptr, b->done_ev.data());
         if (e != cudaSuccess)
             return e;

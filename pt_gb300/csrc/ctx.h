@@ -67,6 +67,7 @@ struct pt_ctx {
     DevBuf<DevMaterial> materials;
     DevBuf<float> material_ior; // refractive extension; meaningful only when has_ior
     bool has_ior = false;
+    bool plain = false; // no material has a map bit or an index of refraction
     DevBuf<uint8_t> texels;
     DevBuf<DevTexture> textures;
     uint32_t texture_count = 0;

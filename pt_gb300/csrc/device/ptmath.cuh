@@ -112,6 +112,21 @@ __device__ __forceinline__ float pt_cos(float x)
     return ((q + 1) & 2) ? -c : c;
 }
 
+// Both at once: one reduction and one evaluation of each polynomial.
+__device__ __forceinline__ void pt_sincos(float x, float& sin_x, float& cos_x)
+{
+    if (!isfinite(x)) {
+        sin_x = cos_x = x - x;
+        return;
+    }
+    int q;
+    const float r = sc::reduce(x, &q);
+    const float sp = sc::sin_poly(r), cp = sc::cos_poly(r);
+    const float s = (q & 1) ? cp : sp, c = (q & 1) ? sp : cp;
+    sin_x = (q & 2) ? -s : s;
+    cos_x = ((q + 1) & 2) ? -c : c;
+}
+
 // ---------------------------------------------------------------- sampler
 // Owen-scrambled Sobol' sampler of shaders/pathtrace/sample.hlsli:94-166
 // (Burley 2020 with the Laine-Karras permutation).  The 4x32 direction
@@ -213,8 +228,10 @@ __device__ __forceinline__ f2 sample_2d(Sampler& s)
 __device__ __forceinline__ f3 cosine_weighted_rand_dir(f2 u)
 {
     float su = sqrtf(u.x);
-    float x = su * pt_cos((2.0f * PI_F) * u.y);
-    float y = su * pt_sin((2.0f * PI_F) * u.y);
+    float sin_phi, cos_phi;
+    pt_sincos((2.0f * PI_F) * u.y, sin_phi, cos_phi);
+    float x = su * cos_phi;
+    float y = su * sin_phi;
     float z = sqrtf(1.0f - u.x);
     return {x, y, z};
 }
@@ -237,7 +254,9 @@ __device__ __forceinline__ f2 sample_concentric_disk(f2 u)
         r = b;
         phi = (PI_F / 2.0f) - (PI_F / 4.0f) * (a / b);
     }
-    return {r * pt_cos(phi), r * pt_sin(phi)};
+    float sin_phi, cos_phi;
+    pt_sincos(phi, sin_phi, cos_phi);
+    return {r * cos_phi, r * sin_phi};
 }
 __device__ __forceinline__ f3 sample_visible_micronormal(f3 v, f2 alpha, f2 u)
 {
@@ -247,8 +266,10 @@ __device__ __forceinline__ f3 sample_visible_micronormal(f3 v, f2 alpha, f2 u)
     float a = 1.0f / (1.0f + v.z);
     float r = sqrtf(u.x);
     float phi = (u.y < a) ? (u.y / a) * PI_F : PI_F + ((u.y - a) / (1.0f - a)) * PI_F;
-    float p1 = r * pt_cos(phi);
-    float p2 = (r * pt_sin(phi)) * ((u.y < a) ? 1.0f : v.z);
+    float sin_phi, cos_phi;
+    pt_sincos(phi, sin_phi, cos_phi);
+    float p1 = r * cos_phi;
+    float p2 = (r * sin_phi) * ((u.y < a) ? 1.0f : v.z);
     float s = sqrtf(fmaxf(0.0f, (1.0f - p1 * p1) - p2 * p2));
     f3 m = (p1 * x + p2 * y) + s * v;
     return normalize(mk3(alpha.x * m.x, alpha.y * m.y, fmaxf(1e-6f, m.z)));
@@ -285,8 +306,20 @@ __device__ __forceinline__ float lambda_fn(f3 m, f2 alpha)
     float alpha2 = sq(cos_phi * alpha.x) + sq(sin_phi * alpha.y);
     return (sqrtf(1.0f + alpha2 * tan2) - 1.0f) / 2.0f;
 }
-__device__ __forceinline__ float g1_fn(f3 v, f2 alpha) { return 1.0f / (1.0f + lambda_fn(v, alpha)); }
-__device__ __forceinline__ float masking(f3 o, f3 i, f2 alpha) { return 1.0f / ((1.0f + lambda_fn(o, alpha)) + lambda_fn(i, alpha)); }
+// The terms of the view direction o, formed once per hit: lambda(o) of the
+// masking terms, and g1(o) / |cos o| of the micronormal density.
+struct ViewTerms {
+    float lambda, g1_over_cos;
+};
+__device__ __forceinline__ ViewTerms view_terms(f3 o, f2 alpha)
+{
+    const float lambda = lambda_fn(o, alpha);
+    return ViewTerms{lambda, (1.0f / (1.0f + lambda)) / fabsf(cos_theta(o))};
+}
+__device__ __forceinline__ float masking(const ViewTerms& view, f3 i, f2 alpha)
+{
+    return 1.0f / ((1.0f + view.lambda) + lambda_fn(i, alpha));
+}
 __device__ __forceinline__ float distribution(f3 m, f2 alpha)
 {
     float tan2 = tan2_theta(m);
@@ -301,13 +334,13 @@ __device__ __forceinline__ float distribution(f3 m, f2 alpha)
 }
 __device__ __forceinline__ float diffuse_sample_probability(float metalness) { return lerpf(0.5f, 0.0f, metalness); }
 
-__device__ __forceinline__ f3 evaluate_brdf(const BrdfInput& in, f3 i, f3 o, f3 m, float& pdf)
+// d = distribution(m, in.alpha)
+__device__ __forceinline__ f3 evaluate_brdf(const BrdfInput& in, const ViewTerms& view, f3 i, f3 o, f3 m, float d, float& pdf)
 {
     f3 f0 = lerp3(in.specular * 0.08f, in.base_colour, in.metalness);
     float cos_d = dot(m, o);
     float f = fresnel_schlick(cos_d);
-    float g = masking(o, i, in.alpha);
-    float d = distribution(m, in.alpha);
+    float g = masking(view, i, in.alpha);
     f3 lf = lerp3(f0, mk3(1.0f, 1.0f, 1.0f), f);
     float denom = (4.0f * cos_theta(i)) * cos_theta(o);
     f3 specular = ((d * lf) * g) / denom;
@@ -317,13 +350,15 @@ __device__ __forceinline__ f3 evaluate_brdf(const BrdfInput& in, f3 i, f3 o, f3 
     // result (pathtrace.ch.hlsl:93-100,114); it is omitted.
     float diffuse_prob = diffuse_sample_probability(in.metalness);
     float pdf_diffuse = cos_theta(i) / PI_F;
-    float pdf_m = ((g1_fn(o, in.alpha) / fabsf(cos_theta(o))) * d) * fabsf(cos_d);
+    float pdf_m = (view.g1_over_cos * d) * fabsf(cos_d);
     float pdf_gtr = pdf_m / (4.0f * fabsf(cos_d));
     pdf = pdf_diffuse * diffuse_prob + pdf_gtr * (1.0f - diffuse_prob);
     return specular + diffuse;
 }
 
-__device__ __forceinline__ f3 sample_direction(f3 o, f2 alpha, float metalness, Sampler& smp, f3& m, float& w, float& pdf)
+// d: distribution(m, alpha) of the sampled micronormal
+__device__ __forceinline__ f3 sample_direction(f3 o, f2 alpha, float metalness, const ViewTerms& view, Sampler& smp, f3& m, float& d,
+                                               float& w, float& pdf)
 {
     f3 i;
     float diffuse_prob = diffuse_sample_probability(metalness);
@@ -338,7 +373,8 @@ __device__ __forceinline__ f3 sample_direction(f3 o, f2 alpha, float metalness, 
     }
     float pdf_diffuse = cos_theta(i) / PI_F;
     float cos_d = dot(m, o);
-    float pdf_m = ((g1_fn(o, alpha) / fabsf(cos_theta(o))) * distribution(m, alpha)) * fabsf(cos_d);
+    d = distribution(m, alpha);
+    float pdf_m = (view.g1_over_cos * d) * fabsf(cos_d);
     float pdf_gtr = pdf_m / (4.0f * fabsf(cos_d));
     pdf_diffuse = pdf_diffuse * diffuse_prob;
     pdf_gtr = pdf_gtr * (1.0f - diffuse_prob);

@@ -111,6 +111,7 @@ struct DevScene {
     int tlas_root;
     f3 env;
     uint32_t* error_word; // bit 0: traversal stack overflow
+    uint32_t plain;       // 1: no material has a map bit, none refracts
 };
 
 constexpr uint32_t ERR_STACK_OVERFLOW = 1u;

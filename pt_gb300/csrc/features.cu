@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(128) k_features(RenderArgs a, float4* feat_a, 
             if (!trace_closest(a.s, ro, rd, a.near_plane, a.far_plane, h, tc))
                 continue;
             f3 ha, hn;
-            hit_features(a.s, h, rd, ha, hn);
+            hit_features<false>(a.s, h, rd, ha, hn);
             alb = alb + ha;
             nrm = nrm + hn;
             depth += h.t;

@@ -97,7 +97,7 @@ struct BatchWave {
 cudaError_t wave_batch_prepare();
 cudaError_t launch_wavefront_batch(const RenderArgs* jobs, const WaveShare* shares, const BatchWave* waves, uint32_t wave_count,
                                    uint32_t* path_share, unsigned long long* counters, void* state, size_t state_bytes,
-                                   uint32_t n_paths_max, bool w4, int sm_count, uint32_t* launches, cudaStream_t stream,
+                                   uint32_t n_paths_max, bool w4, bool plain, int sm_count, uint32_t* launches, cudaStream_t stream,
                                    const WaveMulti& multi, uint32_t* path_share2 = nullptr,
                                    cudaEvent_t* wave_done = nullptr);
 // Records `ev` on `st` so that its time can be read later: inside a stream

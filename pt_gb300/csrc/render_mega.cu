@@ -17,7 +17,7 @@ __device__ __forceinline__ void shade_segment(const DevScene& s, PathState& pl, 
     nee.add = false;
     nee.trace = false;
     NeeKeep keep{nee};
-    shade_hit(s, pl, ro, rd, h, keep);
+    shade_hit<false>(s, pl, ro, rd, h, keep);
     float vis = 0.0f;
     if (nee.trace) {
         shadow_rays++;
@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(128) k_megakernel(RenderArgs a)
             if (a.feat_a) {
                 f3 alb = mk3(0.0f, 0.0f, 0.0f), nrm = alb;
                 if (hit)
-                    hit_features(s, h, rd, alb, nrm);
+                    hit_features<false>(s, h, rd, alb, nrm);
                 feature_mean(fa, make_float4(alb.x, alb.y, alb.z, hit ? h.t : 0.0f), si);
                 feature_mean(fn, make_float4(nrm.x, nrm.y, nrm.z, 0.0f), si);
             }

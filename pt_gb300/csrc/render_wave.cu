@@ -494,7 +494,7 @@ struct NeeToWave {
     }
 };
 
-template <class Src, int MINB>
+template <class Src, int MINB, bool PLAIN>
 __global__ void __launch_bounds__(128, MINB) k_wf_shade(WaveArgs<Src> a, uint32_t qi)
 {
     const uint32_t* qin = a.w.hit_queue;
@@ -541,11 +541,11 @@ __global__ void __launch_bounds__(128, MINB) k_wf_shade(WaveArgs<Src> a, uint32_
                 h.prim = prim;
                 if (sg == 0 && R.feat_a) {
                     f3 alb, nrm;
-                    hit_features(s, h, rd, alb, nrm);
+                    hit_features<PLAIN>(s, h, rd, alb, nrm);
                     a.w.f_a[p] = make_float4(alb.x, alb.y, alb.z, h.t);
                     a.w.f_n[p] = make_float4(nrm.x, nrm.y, nrm.z, 0.0f);
                 }
-                shade_hit(s, pl, ro, rd, h, nee_out);
+                shade_hit<PLAIN>(s, pl, ro, rd, h, nee_out);
             }
             trace = nee_out.traced;
             if (trace)
@@ -1110,11 +1110,22 @@ cudaError_t wave_batch_prepare()
     return cudaGetLastError();
 }
 
+template <class Src, bool PLAIN>
+static void launch_shade(int resident, uint32_t grid, cudaStream_t st, const WaveArgs<Src>& a, uint32_t qi)
+{
+    if (resident == 5)
+        k_wf_shade<Src, 5, PLAIN><<<grid, 128, 0, st>>>(a, qi);
+    else if (resident == 6)
+        k_wf_shade<Src, 6, PLAIN><<<grid, 128, 0, st>>>(a, qi);
+    else
+        k_wf_shade<Src, 0, PLAIN><<<grid, 128, 0, st>>>(a, qi);
+}
+
 // One wave: raygen, (extend, shade, shadow, reset) per segment, accumulate.
 // acc_wait / acc_done (optional) order the accumulation after an earlier
 // wave's on another stream and mark its completion.
 template <class Src>
-static uint32_t launch_wave(const WaveArgs<Src>& a, bool w4, uint32_t max_bounces, uint32_t accum_threads, int sm_count,
+static uint32_t launch_wave(const WaveArgs<Src>& a, bool w4, bool plain, uint32_t max_bounces, uint32_t accum_threads, int sm_count,
                             cudaStream_t st, const ShadowStream& shadow, StageTimer* tm = nullptr,
                             cudaEvent_t acc_wait = nullptr, cudaEvent_t acc_done = nullptr)
 {
@@ -1163,12 +1174,10 @@ static uint32_t launch_wave(const WaveArgs<Src>& a, bool w4, uint32_t max_bounce
         if (sg > 0 && overlap) // the radiance of escaped and shaded paths comes after their light term
             cudaStreamWaitEvent(st, shadow.traced, 0);
         k_wf_split<Src><<<capped_grid(a.src.n_paths, 256, sm_count), 256, 0, st>>>(a, qi);
-        if (sv.shade == 5)
-            k_wf_shade<Src, 5><<<sgrid, 128, 0, st>>>(a, qi);
-        else if (sv.shade == 6)
-            k_wf_shade<Src, 6><<<sgrid, 128, 0, st>>>(a, qi);
+        if (plain)
+            launch_shade<Src, true>(sv.shade, sgrid, st, a, qi);
         else
-            k_wf_shade<Src, 0><<<sgrid, 128, 0, st>>>(a, qi);
+            launch_shade<Src, false>(sv.shade, sgrid, st, a, qi);
         mark(3);
         if (overlap) {
             cudaEventRecord(shadow.shaded, st);
@@ -1241,10 +1250,10 @@ cudaError_t launch_wavefront(const RenderArgs& r, void* state, size_t state_byte
         x.src.first_sample = r.sample_index + done;
         x.src.n_paths = x.src.samples * x.src.pixels;
         if (ways > 1)
-            nl += launch_wave(x, w4, r.max_bounces, x.src.pixels, sm_count, k ? multi.stream[k] : st, multi.shadow[k], nullptr,
+            nl += launch_wave(x, w4, r.s.plain != 0, r.max_bounces, x.src.pixels, sm_count, k ? multi.stream[k] : st, multi.shadow[k], nullptr,
                               w ? multi.acc[(w - 1) % (uint32_t)ways] : nullptr, multi.acc[k]);
         else
-            nl += launch_wave(x, w4, r.max_bounces, x.src.pixels, sm_count, st, timer ? ShadowStream{} : multi.shadow[0], timer);
+            nl += launch_wave(x, w4, r.s.plain != 0, r.max_bounces, x.src.pixels, sm_count, st, timer ? ShadowStream{} : multi.shadow[0], timer);
         done += x.src.samples;
     }
     if (ways > 1) {
@@ -1260,7 +1269,7 @@ cudaError_t launch_wavefront(const RenderArgs& r, void* state, size_t state_byte
 
 cudaError_t launch_wavefront_batch(const RenderArgs* jobs, const WaveShare* shares, const BatchWave* waves, uint32_t wave_count,
                                    uint32_t* path_share, unsigned long long* counters, void* state, size_t state_bytes,
-                                   uint32_t n_paths_max, bool w4, int sm_count, uint32_t* launches, cudaStream_t st,
+                                   uint32_t n_paths_max, bool w4, bool plain, int sm_count, uint32_t* launches, cudaStream_t st,
                                    const WaveMulti& multi, uint32_t* path_share2, cudaEvent_t* wave_done)
 {
     WaveArgs<ManyJobs> a[2];
@@ -1290,10 +1299,10 @@ cudaError_t launch_wavefront_batch(const RenderArgs* jobs, const WaveShare* shar
         x.src.n_pixels = bw.n_pixels;
         const cudaStream_t ws = (ways == 2 && (i & 1)) ? multi.stream[1] : st;
         if (ways == 2)
-            nl += launch_wave(x, w4, bw.max_bounces, bw.n_pixels, sm_count, ws, multi.shadow[i & 1], nullptr,
+            nl += launch_wave(x, w4, plain, bw.max_bounces, bw.n_pixels, sm_count, ws, multi.shadow[i & 1], nullptr,
                               i ? multi.acc[(i - 1) & 1] : nullptr, multi.acc[i & 1]);
         else
-            nl += launch_wave(x, w4, bw.max_bounces, bw.n_pixels, sm_count, ws, multi.shadow[0]);
+            nl += launch_wave(x, w4, plain, bw.max_bounces, bw.n_pixels, sm_count, ws, multi.shadow[0]);
         if (wave_done) // after the wave's accumulation, the last of its launches
             record_timed(wave_done[i], ws);
     }
