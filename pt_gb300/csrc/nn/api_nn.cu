@@ -27,22 +27,22 @@ namespace {
 
 using pt::nn::Act;
 
-// Per-call tensor maps for the single-layer entry points.
-bool map_for(CUtensorMap* tile, CUtensorMap* chunk, const Act& a, std::string& err)
+// Per-call tensor map for the single-layer entry points.
+bool map_for(CUtensorMap* map, const Act& a, int tx, int ty, std::string& err)
 {
-    int tx, ty;
     const char* why = nullptr;
-    pt::nn::conv_tile_shape(a.w, tx, ty);
-    if (tile && !pt::nn::encode_act_map(tile, a, tx, ty, &why)) {
-        err = why;
-        return false;
-    }
-    pt::nn::wgrad_chunk_shape(a.w, tx, ty);
-    if (chunk && !pt::nn::encode_act_map(chunk, a, tx, ty, &why)) {
+    if (!pt::nn::encode_act_map(map, a, tx, ty, &why)) {
         err = why;
         return false;
     }
     return true;
+}
+
+bool tile_map_for(CUtensorMap* tile, const Act& a, std::string& err)
+{
+    int tx, ty;
+    pt::nn::conv_tile_shape(a.w, tx, ty);
+    return map_for(tile, a, tx, ty, err);
 }
 
 thread_local std::string g_layer_error;
@@ -277,7 +277,7 @@ int pt_nn_conv3x3(const uint16_t* in, uint32_t n, uint32_t h, uint32_t w, uint32
     a.w = (int)w;
     a.pitch = (int)in_pitch;
     CUtensorMap tile;
-    if (!map_for(&tile, nullptr, a, g_layer_error))
+    if (!tile_map_for(&tile, a, g_layer_error))
         return PT_ERR_INVALID;
     const bool rows = pt::nn::use_rows_kernel();
     if ((rows ? pt::nn::pack_weights_rows(weights, (int)c_in, (int)c_out, s.fwd, s.bwd, st)
@@ -316,7 +316,7 @@ int pt_nn_conv3x3_dgrad(const uint16_t* grad_out, uint32_t n, uint32_t h, uint32
     g.w = (int)w;
     g.pitch = (int)c_out;
     CUtensorMap tile;
-    if (!map_for(&tile, nullptr, g, g_layer_error))
+    if (!tile_map_for(&tile, g, g_layer_error))
         return PT_ERR_INVALID;
     const bool rows = pt::nn::use_rows_kernel();
     if ((rows ? pt::nn::pack_weights_rows(weights, (int)c_in, (int)c_out, s.fwd, s.bwd, st)
@@ -359,7 +359,8 @@ int pt_nn_conv3x3_wgrad(const uint16_t* in, uint32_t n, uint32_t h, uint32_t w, 
     g.p = const_cast<uint16_t*>(grad_out);
     g.pitch = (int)c_out;
     CUtensorMap xc, gc;
-    if (!map_for(nullptr, &xc, x, g_layer_error) || !map_for(nullptr, &gc, g, g_layer_error))
+    const int tx = pt::nn::wgrad_tile_width((int)w);
+    if (!map_for(&xc, x, tx + 2, 1, g_layer_error) || !map_for(&gc, g, tx, 1, g_layer_error))
         return PT_ERR_INVALID;
     const int sms = sm_count();
     pt::nn::WgradCall c{};

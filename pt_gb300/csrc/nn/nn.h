@@ -24,9 +24,10 @@ struct Act {
 // pixels of one image.  False (and a message in *why) on failure.
 bool encode_act_map(CUtensorMap* map, const Act& a, int tx, int ty, const char** why);
 
-// Tile shapes: conv tiles hold 128 pixels, weight-gradient chunks 64.
+// Tile shapes: conv tiles hold 128 pixels; weight-gradient chunks are rows of
+// wgrad_tile_width pixels.
 void conv_tile_shape(int w, int& tx, int& ty);
-void wgrad_chunk_shape(int w, int& tx, int& ty);
+int wgrad_tile_width(int w);
 
 // Packed weight sizes (elements) of one layer.
 inline size_t packed_elems(int cin, int cout) { return (size_t)9 * cin * cout; }
@@ -67,7 +68,8 @@ cudaError_t conv3x3_rows(const ConvCall& c, const CUtensorMap* halo_map, int sm_
 bool use_rows_kernel();
 
 // dw[tap][ci][co] += sum_p x[p + offset(tap)][x_c0 + ci] * g[p][g_c0 + co]
-// over all pixels (dw must be zeroed by the caller).  Maps use the wgrad box.
+// over all pixels (dw must be zeroed by the caller).  x_map has a box of
+// wgrad_tile_width + 2 pixels of one row, g_map one of wgrad_tile_width.
 struct WgradCall {
     const CUtensorMap* x_map;
     int x_c0, cin;

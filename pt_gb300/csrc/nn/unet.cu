@@ -126,8 +126,8 @@ bool UNet::make(Buf& b, int level, int channels, std::string& err)
         err = why;
         return false;
     }
-    wgrad_chunk_shape(b.a.w, tx, ty);
-    if (!encode_act_map(&b.chunk, b.a, tx, ty, &why)) {
+    tx = wgrad_tile_width(b.a.w);
+    if (!encode_act_map(&b.wg_x, b.a, tx + 2, 1, &why) || !encode_act_map(&b.wg_g, b.a, tx, 1, &why)) {
         err = why;
         return false;
     }
@@ -350,10 +350,10 @@ cudaError_t UNet::dgrad(int l, Buf& g, Buf& out, const Buf* mask, int mask_c0, c
 cudaError_t UNet::wgrad(int l, Buf& x, int x_c0, Buf& g, cudaStream_t st)
 {
     WgradCall c{};
-    c.x_map = &x.chunk;
+    c.x_map = &x.wg_x;
     c.x_c0 = x_c0;
     c.cin = LAYERS[l].cin;
-    c.g_map = &g.chunk;
+    c.g_map = &g.wg_g;
     c.g_c0 = 0;
     c.cout = LAYERS[l].cout;
     c.n = g.a.n;

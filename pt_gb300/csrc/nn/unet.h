@@ -69,7 +69,7 @@ class UNet {
 
     struct Buf {
         Act a;
-        CUtensorMap tile, chunk;
+        CUtensorMap tile, wg_x, wg_g; // weight gradient: as the layer's input, as its output gradient
         CUtensorMap halo[4]; // halo boxes for 1, 2, 4 and 8 rows per tile
     };
 
