@@ -303,18 +303,19 @@ __global__ void __launch_bounds__(128) k_wgrad(const __grid_constant__ CUtensorM
             }
             tc_fence_after();
             const uint32_t sa = smem_addr(smem + (size_t)s * stage_bytes);
-            const uint32_t sb = sa + a_bytes;
-            for (int y = 0; y < p.ry; y++)
-                for (int ks = 0; ks < p.tx / 16; ks++) {
-                    // MN-major, no swizzle: lbo = 128 between 8-pixel groups of K,
-                    // sbo between 8-channel groups of M/N
-                    const uint64_t bd = smem_desc(sb + (uint32_t)y * g_row + (uint32_t)ks * 256u, 128u, g_group);
-                    for (int t = 0; t < nt; t++) {
-                        const uint32_t a0 = sa + (uint32_t)t * tile_bytes + (uint32_t)y * input_row + (uint32_t)ks * 256u;
+            // MN-major, no swizzle: lbo = 128 between 8-pixel groups of K, sbo
+            // between 8-channel groups of M/N.  A step of a descriptor's address
+            // is 16 bytes: one pixel.
+            uint64_t ad_y = smem_desc(sa, 128u, p.row_bytes);
+            uint64_t bd = smem_desc(sa + a_bytes, 128u, g_group);
+            for (int y = 0; y < p.ry; y++, ad_y += input_row >> 4)
+                for (int ks = 0; ks < p.tx / 16; ks++, bd += 16) {
+                    uint64_t ad = ad_y + 16u * (uint32_t)ks;
+                    uint32_t d = tmem;
+                    for (int t = 0; t < nt; t++, ad += tile_bytes >> 4, d += 3u * (uint32_t)p.cout) {
 #pragma unroll
                         for (int kx = 0; kx < 3; kx++)
-                            mma_bf16(tmem + (uint32_t)((t * 3 + kx) * p.cout), smem_desc(a0 + (uint32_t)kx * 16u, 128u, p.row_bytes), bd,
-                                     idesc, (i | y | ks) != 0);
+                            mma_bf16(d + (uint32_t)(kx * p.cout), ad + kx, bd, idesc, (i | y | ks) != 0);
                     }
                 }
             mma_commit(&empty[s]);

@@ -134,6 +134,7 @@ __global__ void __launch_bounds__(192) k_conv3x3_rows(const __grid_constant__ CU
         if (lane == 0) {
             const uint32_t idesc = idesc_bf16(128, (uint32_t)p.nout, false, false);
             const uint32_t b_lbo = (uint32_t)p.nout * 16;
+            const uint32_t b_step = b_tap >> 4;
             uint32_t it = 0, tc = 0;
             for (int t = blockIdx.x; t < p.tiles && !failed(fail); t += gridDim.x, tc++) {
                 // buffer b's previous tile (two tiles back) must have been drained
@@ -152,15 +153,14 @@ __global__ void __launch_bounds__(192) k_conv3x3_rows(const __grid_constant__ CU
                     }
                     tc_fence_after();
                     const uint32_t sa = smem_addr(smem + (size_t)s * stage_bytes);
-                    const uint32_t sb = sa + a_bytes;
-                    for (int r = 0; r < MT; r++) {
-                        for (int tap = 0; tap < 9; tap++) {
-                            const int ky = tap / 3, kx = tap % 3;
-                            const uint32_t a_off = (uint32_t)((r + ky) * HALO_W + kx) * 16u;
-                            const uint64_t ad = smem_desc(sa + a_off, a_box, 128u);
-                            const uint64_t bd = smem_desc(sb + (uint32_t)tap * b_tap, b_lbo, 128u);
-                            mma_bf16(acc + (uint32_t)(r * p.nout), ad, bd, idesc, (c | tap) != 0);
-                        }
+                    const uint64_t bd = smem_desc(sa + a_bytes, b_lbo, 128u);
+                    uint64_t ad = smem_desc(sa, a_box, 128u);
+                    uint32_t d = acc;
+                    // a step of a descriptor's address is 16 bytes: one pixel of the halo
+                    for (int r = 0; r < MT; r++, ad += HALO_W, d += p.nout) {
+#pragma unroll
+                        for (int tap = 0; tap < 9; tap++)
+                            mma_bf16(d, ad + (uint32_t)(tap / 3 * HALO_W + tap % 3), bd + (uint32_t)tap * b_step, idesc, (c | tap) != 0);
                     }
                     mma_commit(&empty[s]);
                 }
