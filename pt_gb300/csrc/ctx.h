@@ -27,16 +27,20 @@ using pt::DevTexture;
 using pt::REF_EMPTY;
 using pt::TriRec;
 
-// One device allocation; released explicitly or by the owning context.
+// One device allocation; released explicitly or by the owning context.  Asking
+// for the size it has keeps it (a scene loaded again: cudaMalloc and cudaFree
+// of the large arrays took 0.9 ms of a two-million-triangle scene's load).
 template <typename T>
 struct DevBuf {
     T* p = nullptr;
     size_t n = 0;
     cudaError_t alloc(size_t count)
     {
-        release();
         if (count == 0)
             count = 1;
+        if (p && n == count)
+            return cudaSuccess;
+        release();
         cudaError_t e = cudaMalloc((void**)&p, count * sizeof(T));
         if (e != cudaSuccess) {
             p = nullptr;
@@ -73,6 +77,8 @@ struct pt_ctx {
     uint32_t texture_count = 0;
     DevBuf<uint32_t> light;
     DevBuf<uint32_t> mesh_vertex_offset, mesh_index_offset, mesh_tri_base, inst_mesh;
+    DevBuf<pt_mesh_range> mesh_ranges; // as uploaded, for the check of the indices
+    DevBuf<uint32_t> scene_check;      // first non-finite vertex, first mesh with an index outside its vertices
     DevBuf<DevInstance> dinst;
     uint32_t vertex_count = 0, index_count = 0, mesh_count = 0, tri_count = 0, instance_count = 0, material_count = 0;
     uint32_t light_words = 0, light_count = 0;
