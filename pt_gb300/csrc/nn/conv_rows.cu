@@ -11,10 +11,18 @@
 // TMEM.
 //
 // Warp roles: warp 0 produces (TMA), warp 1 allocates TMEM and issues the
-// MMAs, warps 2-5 drain the accumulators (bias, ReLU, gradient mask, store).
+// MMAs, warps 2-9 drain the accumulators (bias, ReLU, gradient mask, store).
 // One persistent CTA per SM with as many pipeline stages as shared memory
 // holds; the accumulators are double-buffered in TMEM (2 x MT x N columns),
 // so the MMAs of the next tile run while the epilogue drains this one.
+//
+// With few output channels a multiplication is bound by its A operand (128
+// pixels, 32 cycles against 16 of arithmetic at N = 32) and by its issue, and
+// the drain by its memory instructions.  So the three row taps that a shifted
+// halo row is multiplied by follow each other and share it (tc.cuh), the
+// issuing warp's loop is uniform, and eight warps drain with the bias in shared
+// memory and a 32-byte access per 16 channels.  At 1080 x 1920: layer 96 -> 32
+// 200 -> 147 us (813 TFLOP/s), 16 -> 32 77 -> 47, all 15 layers 1,130 -> 775 us.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -30,6 +38,8 @@ namespace {
 
 constexpr int HALO_W = 130; // 128 pixels + one on each side
 constexpr int KC = 16;      // input channels per pipeline stage
+constexpr int EPILOGUE_WARPS = 8;
+constexpr int ROWS_THREADS = 64 + 32 * EPILOGUE_WARPS;
 
 struct RowsParams {
     int cin, c0, nout, mt;
@@ -45,6 +55,7 @@ struct RowsParams {
     int n, h, w, tiles_x, tiles_y, tiles;
     int stages;
     uint32_t tmem_cols; // one accumulator buffer; the CTA allocates two
+    int wide;           // out and mask rows are 32-byte aligned
     uint32_t* error;
 };
 
@@ -64,7 +75,112 @@ __device__ __forceinline__ bool failed(volatile uint32_t* fail)
     return *fail != 0;
 }
 
-__global__ void __launch_bounds__(192) k_conv3x3_rows(const __grid_constant__ CUtensorMap amap, RowsParams p)
+// Bias, ReLU, gradient mask, residual base and store of 16 output channels
+// (unit j) of pixel (px, py).
+__device__ __forceinline__ void finish_unit(const RowsParams& p, const float* s_bias, const uint32_t (&v32)[16], int img, int py, int px, int j)
+{
+    if (px >= p.w || py >= p.h)
+        return;
+    const size_t pix = ((size_t)img * p.h + py) * p.w + px;
+    float v[16];
+#pragma unroll
+    for (int k = 0; k < 16; k += 4) {
+        const float4 b = *reinterpret_cast<const float4*>(s_bias + j * 16 + k);
+        v[k] = __uint_as_float(v32[k]);
+        v[k + 1] = __uint_as_float(v32[k + 1]);
+        v[k + 2] = __uint_as_float(v32[k + 2]);
+        v[k + 3] = __uint_as_float(v32[k + 3]);
+        if (p.bias) {
+            v[k] += b.x;
+            v[k + 1] += b.y;
+            v[k + 2] += b.z;
+            v[k + 3] += b.w;
+        }
+    }
+    if (p.relu) {
+#pragma unroll
+        for (int k = 0; k < 16; k++)
+            v[k] = fmaxf(v[k], 0.0f);
+    }
+    if (p.mask) {
+        const uint16_t* mp = p.mask + pix * p.mask_pitch + p.mask_c0 + j * 16;
+        uint32_t mw[8];
+        if (p.wide) {
+            load32(mp, mw);
+        } else {
+            const uint4 q0 = reinterpret_cast<const uint4*>(mp)[0], q1 = reinterpret_cast<const uint4*>(mp)[1];
+            mw[0] = q0.x, mw[1] = q0.y, mw[2] = q0.z, mw[3] = q0.w, mw[4] = q1.x, mw[5] = q1.y, mw[6] = q1.z, mw[7] = q1.w;
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            if (!bf16_pos((uint16_t)(mw[k] & 0xFFFFu)))
+                v[2 * k] = 0.0f;
+            if (!bf16_pos((uint16_t)(mw[k] >> 16)))
+                v[2 * k + 1] = 0.0f;
+        }
+    }
+    if (p.out_f32) {
+        if (p.residual && j == 0) {
+            const float4 r4 = *reinterpret_cast<const float4*>(p.residual + pix * 4);
+            v[0] += r4.x;
+            v[1] += r4.y;
+            v[2] += r4.z;
+            v[3] += r4.w;
+        }
+        float* o = p.out_f32 + pix * p.out_pitch + j * 16;
+        if (p.wide) {
+#pragma unroll
+            for (int k = 0; k < 16; k += 8) {
+                const uint32_t w[8] = {__float_as_uint(v[k]),     __float_as_uint(v[k + 1]), __float_as_uint(v[k + 2]), __float_as_uint(v[k + 3]),
+                                       __float_as_uint(v[k + 4]), __float_as_uint(v[k + 5]), __float_as_uint(v[k + 6]), __float_as_uint(v[k + 7])};
+                store32(o + k, w);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                reinterpret_cast<float4*>(o)[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+        }
+        return;
+    }
+    uint16_t* o = p.out + pix * p.out_pitch + p.out_c0 + j * 16;
+    uint32_t w[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+        w[k] = pack2(v[2 * k], v[2 * k + 1]);
+    if (p.wide) {
+        store32(o, w);
+    } else {
+        reinterpret_cast<uint4*>(o)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        reinterpret_cast<uint4*>(o)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    }
+}
+
+// One input row's multiplications of a slice: for each column tap the row taps
+// LO..HI, which share the A operand and go to the accumulators of HI - LO + 1
+// output rows (d: the one of row tap 0).  An output row's products are still
+// added tap by tap in the order of the weights.  `more`: not the first slice.
+template <int LO, int HI>
+__device__ __forceinline__ void input_row(uint32_t d, uint64_t ad, uint64_t bd, int nout, uint32_t b_step, uint32_t idesc, bool more)
+{
+#pragma unroll
+    for (int kx = 0; kx < 3; kx++)
+#pragma unroll
+        for (int ky = LO; ky <= HI; ky++) {
+            const uint32_t to = d - (uint32_t)(ky * nout);
+            const uint64_t b = bd + (uint32_t)(3 * ky + kx) * b_step;
+            const bool add = ky > 0 || kx > 0 || more; // the first product of an output row starts its accumulator
+            if (LO == HI)
+                mma_bf16_warp<DISCARD>(to, ad + kx, b, idesc, add);
+            else if (ky == LO)
+                mma_bf16_warp<FILL>(to, ad + kx, b, idesc, add);
+            else if (ky == HI)
+                mma_bf16_warp<LAST_USE>(to, ad + kx, b, idesc, add);
+            else
+                mma_bf16_warp<USE>(to, ad + kx, b, idesc, add);
+        }
+}
+
+__global__ void __launch_bounds__(ROWS_THREADS) k_conv3x3_rows(const __grid_constant__ CUtensorMap amap, RowsParams p)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     const int MT = p.mt;
@@ -82,9 +198,12 @@ __global__ void __launch_bounds__(192) k_conv3x3_rows(const __grid_constant__ CU
     uint64_t* acc_empty = acc_full + 2; // [2]: buffer b was drained
     uint32_t* tslot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile uint32_t* fail = tslot + 1;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float* s_bias = reinterpret_cast<float*>(((uintptr_t)(tslot + 2) + 15) & ~(uintptr_t)15); // zeros without a bias
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31; // warp: uniform for the compiler too
     const int chunks = p.cin / KC;
 
+    for (int k = threadIdx.x; k < p.nout; k += ROWS_THREADS)
+        s_bias[k] = p.bias ? p.bias[k] : 0.0f;
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; s++) {
             mbar_init(&full[s], 1);
@@ -92,7 +211,7 @@ __global__ void __launch_bounds__(192) k_conv3x3_rows(const __grid_constant__ CU
         }
         for (int b = 0; b < 2; b++) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 4);
+            mbar_init(&acc_empty[b], EPILOGUE_WARPS);
         }
         *fail = 0;
         mbar_init_fence();
@@ -131,46 +250,61 @@ __global__ void __launch_bounds__(192) k_conv3x3_rows(const __grid_constant__ CU
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = idesc_bf16(128, (uint32_t)p.nout, false, false);
-            const uint32_t b_lbo = (uint32_t)p.nout * 16;
-            const uint32_t b_step = b_tap >> 4;
-            uint32_t it = 0, tc = 0;
-            for (int t = blockIdx.x; t < p.tiles && !failed(fail); t += gridDim.x, tc++) {
-                // buffer b's previous tile (two tiles back) must have been drained
-                const uint32_t b = tc & 1u, use = tc >> 1;
-                if (use > 0 && !mbar_wait(&acc_empty[b], (use - 1) & 1u)) {
+        // the whole warp, one elected lane issuing; every wait's outcome is made uniform
+        const uint32_t idesc = idesc_bf16(128, (uint32_t)p.nout, false, false);
+        const uint32_t b_lbo = (uint32_t)p.nout * 16;
+        const uint32_t b_step = b_tap >> 4;
+        const uint32_t tm = __reduce_or_sync(0xffffffffu, tmem); // in a uniform register
+        uint32_t it = 0, tc = 0;
+        for (int t = blockIdx.x; t < p.tiles; t += gridDim.x, tc++) {
+            // buffer b's previous tile (two tiles back) must have been drained
+            const uint32_t b = tc & 1u, use = tc >> 1;
+            const bool ready = !failed(fail) && (use == 0 || mbar_wait(&acc_empty[b], (use - 1) & 1u));
+            if (!__all_sync(0xffffffffu, ready)) {
+                if (lane == 0)
                     atomicOr((uint32_t*)fail, 1u);
+                break;
+            }
+            tc_fence_after();
+            const uint32_t acc = tm + b * p.tmem_cols;
+            for (int c = 0; c < chunks; c++, it++) {
+                const uint32_t s = it % S;
+                if (!__all_sync(0xffffffffu, mbar_wait(&full[s], (it / S) & 1u))) {
+                    if (lane == 0)
+                        atomicOr((uint32_t*)fail, 1u);
                     break;
                 }
                 tc_fence_after();
-                const uint32_t acc = tmem + b * p.tmem_cols;
-                for (int c = 0; c < chunks; c++, it++) {
-                    const uint32_t s = it % S;
-                    if (!mbar_wait(&full[s], (it / S) & 1u)) {
-                        atomicOr((uint32_t*)fail, 1u);
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t sa = smem_addr(smem + (size_t)s * stage_bytes);
-                    const uint64_t bd = smem_desc(sa + a_bytes, b_lbo, 128u);
-                    uint64_t ad = smem_desc(sa, a_box, 128u);
-                    uint32_t d = acc;
-                    // a step of a descriptor's address is 16 bytes: one pixel of the halo
-                    for (int r = 0; r < MT; r++, ad += HALO_W, d += p.nout) {
-#pragma unroll
-                        for (int tap = 0; tap < 9; tap++)
-                            mma_bf16(d, ad + (uint32_t)(tap / 3 * HALO_W + tap % 3), bd + (uint32_t)tap * b_step, idesc, (c | tap) != 0);
-                    }
-                    mma_commit(&empty[s]);
+                const uint32_t sa = smem_addr(smem) + s * stage_bytes;
+                const uint64_t bd = smem_desc(sa + a_bytes, b_lbo, 128u);
+                uint64_t ad = smem_desc(sa, a_box, 128u);
+                // input row i feeds output rows i, i - 1, i - 2 with the row taps ky = 0, 1, 2
+                for (int i = 0; i < MT + 2; i++, ad += HALO_W) {
+                    const int lo = i < MT ? 0 : i - MT + 1, hi = i < 2 ? i : 2;
+                    const uint32_t d = acc + (uint32_t)(i * p.nout);
+                    if (lo == 0 && hi == 2)
+                        input_row<0, 2>(d, ad, bd, p.nout, b_step, idesc, c != 0);
+                    else if (lo == 0 && hi == 1)
+                        input_row<0, 1>(d, ad, bd, p.nout, b_step, idesc, c != 0);
+                    else if (lo == 0)
+                        input_row<0, 0>(d, ad, bd, p.nout, b_step, idesc, c != 0);
+                    else if (lo == 1 && hi == 2)
+                        input_row<1, 2>(d, ad, bd, p.nout, b_step, idesc, c != 0);
+                    else if (lo == 1)
+                        input_row<1, 1>(d, ad, bd, p.nout, b_step, idesc, c != 0);
+                    else
+                        input_row<2, 2>(d, ad, bd, p.nout, b_step, idesc, c != 0);
                 }
-                mma_commit(&acc_full[b]);
+                mma_commit_warp(&empty[s]);
             }
+            mma_commit_warp(&acc_full[b]);
         }
     } else {
-        // epilogue warps 2..5 drain TMEM lanes 32 * (warp % 4) ..
-        const int quarter = warp & 3;
+        // epilogue warps: two to each quarter of the TMEM lanes (32 * (warp % 4)),
+        // taking the 16-column units of the tile's rows in turn
+        const int quarter = warp & 3, half = (warp - 2) >> 2;
         const int m = quarter * 32 + lane;
+        const int per_row = p.nout / 16, units = MT * per_row;
         uint32_t tc = 0;
         for (int t = blockIdx.x; t < p.tiles; t += gridDim.x, tc++) {
             const uint32_t b = tc & 1u, use = tc >> 1;
@@ -188,53 +322,19 @@ __global__ void __launch_bounds__(192) k_conv3x3_rows(const __grid_constant__ CU
             const int tyi = q % p.tiles_y;
             const int img = q / p.tiles_y;
             const int px = txi * 128 + m;
-            for (int r = 0; r < MT; r++) {
-                const int py = tyi * MT + r;
-                const bool valid = px < p.w && py < p.h;
-                const size_t pix = ((size_t)img * p.h + py) * p.w + px;
-                for (int j = 0; j < p.nout / 16; j++) {
-                    uint32_t v32[16];
-                    tmem_ld16(tmem + b * p.tmem_cols + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(r * p.nout + j * 16), v32);
-                    if (!valid)
-                        continue;
-                    float v[16];
-#pragma unroll
-                    for (int k = 0; k < 16; k++) {
-                        v[k] = __uint_as_float(v32[k]);
-                        if (p.bias)
-                            v[k] += p.bias[j * 16 + k];
-                        if (p.relu)
-                            v[k] = fmaxf(v[k], 0.0f);
-                    }
-                    if (p.mask) {
-                        const uint4* mp = reinterpret_cast<const uint4*>(p.mask + pix * p.mask_pitch + p.mask_c0 + j * 16);
-                        const uint4 q0 = mp[0], q1 = mp[1];
-                        const uint32_t mw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-#pragma unroll
-                        for (int k = 0; k < 8; k++) {
-                            if (!bf16_pos((uint16_t)(mw[k] & 0xFFFFu)))
-                                v[2 * k] = 0.0f;
-                            if (!bf16_pos((uint16_t)(mw[k] >> 16)))
-                                v[2 * k + 1] = 0.0f;
-                        }
-                    }
-                    if (p.out_f32) {
-                        if (p.residual && j == 0) {
-                            const float4 r4 = *reinterpret_cast<const float4*>(p.residual + pix * 4);
-                            v[0] += r4.x;
-                            v[1] += r4.y;
-                            v[2] += r4.z;
-                            v[3] += r4.w;
-                        }
-                        float4* o = reinterpret_cast<float4*>(p.out_f32 + pix * p.out_pitch + j * 16);
-#pragma unroll
-                        for (int k = 0; k < 4; k++)
-                            o[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-                    } else {
-                        uint4* o = reinterpret_cast<uint4*>(p.out + pix * p.out_pitch + p.out_c0 + j * 16);
-                        o[0] = make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
-                        o[1] = make_uint4(pack2(v[8], v[9]), pack2(v[10], v[11]), pack2(v[12], v[13]), pack2(v[14], v[15]));
-                    }
+            const uint32_t from = tmem + b * p.tmem_cols + ((uint32_t)(quarter * 32) << 16);
+            // two units at a time: the second's TMEM read passes while the first is stored
+            for (int u = 2 * half; u < units; u += 4) {
+                uint32_t v0[16], v1[16];
+                const bool two = u + 1 < units;
+                tmem_ld16_issue(from + (uint32_t)(u * 16), v0);
+                if (two)
+                    tmem_ld16_issue(from + (uint32_t)((u + 1) * 16), v1);
+                tmem_ld_wait(v0);
+                finish_unit(p, s_bias, v0, img, tyi * MT + u / per_row, px, u % per_row);
+                if (two) {
+                    tmem_ld_wait(v1);
+                    finish_unit(p, s_bias, v1, img, tyi * MT + (u + 1) / per_row, px, (u + 1) % per_row);
                 }
             }
             tc_fence_before();
@@ -339,7 +439,10 @@ cudaError_t conv3x3_rows(const ConvCall& c, const CUtensorMap* halo_map, int sm_
         return cudaSuccess;
     const size_t a_box = ((size_t)(p.mt + 2) * HALO_W * 16 + 127) & ~(size_t)127;
     const size_t stage = 2 * a_box + (size_t)9 * p.nout * 32;
-    const size_t extra = 8 * (2 * 8 + 4) + 64;
+    const size_t extra = 8 * (2 * 8 + 4) + 64 + 4 * (size_t)p.nout;
+    auto aligned32 = [](const void* q, int pitch, int c0) { return (((uintptr_t)q + 2 * (size_t)c0) & 31) == 0 && pitch % 16 == 0; };
+    const bool out_aligned = p.out_f32 ? ((uintptr_t)p.out_f32 & 31) == 0 && p.out_pitch % 8 == 0 : aligned32(p.out, p.out_pitch, p.out_c0);
+    p.wide = out_aligned && (!p.mask || aligned32(p.mask, p.mask_pitch, p.mask_c0)) ? 1 : 0;
     const size_t smem_max = 232448; // one CTA per SM: all of its shared memory
     int S = 8;
     while (S > 2 && S * stage + extra > smem_max)
@@ -359,7 +462,7 @@ cudaError_t conv3x3_rows(const ConvCall& c, const CUtensorMap* halo_map, int sm_
     }
     // one CTA per SM (its two accumulator buffers may take all 512 TMEM columns)
     const int grid = std::min(p.tiles, sm_count);
-    k_conv3x3_rows<<<grid, 192, smem, st>>>(*halo_map, p);
+    k_conv3x3_rows<<<grid, ROWS_THREADS, smem, st>>>(*halo_map, p);
     return cudaGetLastError();
 }
 

@@ -139,6 +139,47 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint6
                  : "memory");
 }
 
+// The same for a whole converged warp, of which one elected lane (the same
+// every time) issues: the loop around it stays uniform, and a
+// multiplication takes 25 cycles to issue instead of 45.  COLLECT says what
+// happens to the A operand in the tensor core's collector buffer: kept for the
+// next ones (FILL), taken from there (USE), taken for the last time (LAST_USE),
+// or neither.  Reading A (128 rows, 32 cycles) is most of a multiplication by
+// few columns: measured per multiplication with N = 16, 32, 64, 96: 39, 40, 48
+// and 56 cycles, and 20, 25, 36 and 48 when three share A.
+enum Collect { DISCARD, FILL, USE, LAST_USE };
+
+template <Collect COLLECT>
+__device__ __forceinline__ void mma_bf16_warp(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
+{
+#define PT_MMA_WARP(OP)                                                             \
+    asm volatile("{\n\t.reg .pred p, q;\n\t"                                       \
+                 "elect.sync _|q, 0xffffffff;\n\t"                                  \
+                 "setp.ne.b32 p, %4, 0;\n\t"                                        \
+                 "@q tcgen05.mma.cta_group::1.kind::f16.collector::a::" OP          \
+                 " [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),                        \
+                 "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)              \
+                 : "memory")
+    if (COLLECT == FILL)
+        PT_MMA_WARP("fill");
+    else if (COLLECT == USE)
+        PT_MMA_WARP("use");
+    else if (COLLECT == LAST_USE)
+        PT_MMA_WARP("lastuse");
+    else
+        PT_MMA_WARP("discard");
+#undef PT_MMA_WARP
+}
+
+// mma_commit for multiplications issued by mma_bf16_warp.
+__device__ __forceinline__ void mma_commit_warp(uint64_t* bar)
+{
+    asm volatile("{\n\t.reg .pred q;\n\t"
+                 "elect.sync _|q, 0xffffffff;\n\t"
+                 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_addr(bar))
+                 : "memory");
+}
+
 // Arrives on `bar` once every tcgen05 operation this thread issued is done.
 __device__ __forceinline__ void mma_commit(uint64_t* bar)
 {
@@ -147,15 +188,43 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar)
 }
 
 // 32 TMEM lanes x 16 columns of 32 bits: lane i of the warp receives TMEM lane
-// (lane base + i), columns [col, col + 16).  Warp-collective.
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16])
+// (lane base + i), columns [col, col + 16).  Warp-collective; the values are
+// there after tmem_ld_wait, which ties them so that none is used before.
+__device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&r)[16])
 {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
                  "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
                    "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                  : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[16])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
+                   "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+                 :
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16])
+{
+    tmem_ld16_issue(taddr, r);
+    tmem_ld_wait(r);
+}
+
+// 32 bytes (32-byte aligned) by one access.
+__device__ __forceinline__ void store32(void* p, const uint32_t (&v)[8])
+{
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
+                 "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+__device__ __forceinline__ void load32(const void* p, uint32_t (&v)[8])
+{
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "l"(p)
+                 : "memory");
 }
 
 } // namespace nn
