@@ -360,7 +360,7 @@ int pt_nn_conv3x3_wgrad(const uint16_t* in, uint32_t n, uint32_t h, uint32_t w, 
     g.pitch = (int)c_out;
     CUtensorMap xc, gc;
     const int tx = pt::nn::wgrad_tile_width((int)w);
-    if (!map_for(&xc, x, tx + 2, 1, g_layer_error) || !map_for(&gc, g, tx, 1, g_layer_error))
+    if (!map_for(&xc, x, tx, 1, g_layer_error) || !map_for(&gc, g, tx + 2, 1, g_layer_error))
         return PT_ERR_INVALID;
     const int sms = sm_count();
     pt::nn::WgradCall c{};

@@ -199,6 +199,8 @@ __global__ void __launch_bounds__(128) k_conv3x3(const __grid_constant__ CUtenso
         atomicOr(p.error, 1u);
 }
 
+constexpr int WGRAD_LANE_LOADS = 8; // TMA loads of a chunk: at most 32 times as many
+
 struct WgradParams {
     int cin, x_c0, cout, g_c0;
     int groups;        // cin / 8 channel groups
@@ -206,24 +208,27 @@ struct WgradParams {
     int tiles, tiles_per_cta;
     int h, w, tx, ry, chunks_x, chunks_y, chunks, chunks_per_cta; // a chunk: ry rows of tx pixels
     int stages;
-    uint32_t row_bytes; // shared-memory stride of one row of tx + 2 pixels x 8 channels
+    uint32_t row_bytes;   // shared-memory stride of one input row of tx pixels x 8 channels
+    uint32_t g_row_bytes; // and of one gradient row of tx + 2 pixels x 8 channels
     uint32_t tmem_cols;
     float* dw;
     uint32_t* error;
 };
 
-// Weight gradient.  For one column tap kx, the rows of M are (ky, input
-// channel): a chunk's ry + 2 input rows lie in shared memory as [row][group of 8
-// channels][pixel], so the M operand of output row y is 3 nc row groups a fixed
-// stride apart that begin at input row y, and column tap kx begins 16 kx bytes
-// later.  An input pixel is loaded (ry + 2) / ry times instead of nine; what
-// bounds the kernel is the rate at which TMA delivers 16-byte rows (about one a
+// Weight gradient.  The rows of M are (ky, input channel): a chunk's ry + 2
+// input rows lie in shared memory as [row][group of 8 channels][pixel], so the M
+// operand of output row y is 3 nc row groups a fixed stride apart that begin at
+// input row y.  The column taps shift the output gradient instead (dw[kx] = sum
+// over input pixels x of in(x) g(x - kx + 1)): its rows carry a pixel on either
+// side, column tap kx begins (2 - kx) pixels in, and the three multiplications
+// share the M operand.  An input pixel is loaded (ry + 2) / ry times instead of nine; what
+// bounds the kernel is the rate at which TMA delivers 16-byte rows (about 0.8 a
 // cycle and SM).  An M tile holds up to five channel groups (120 of 128 rows);
 // the rest of its rows read whatever follows and are not stored.  A CTA keeps
 // tiles_per_cta x 3 accumulators in TMEM, so that it reads the output gradient
 // once for all of them.  Training batch of 16 x 256 x 256, all 15 layers: 3,070 us
-// with nine shifted loads of each input pixel, 958 so (layer 96 -> 32 at 256 x 256
-// 169 us, 57 GFLOP; 32 -> 32 79 us).
+// with nine shifted loads of each input pixel, 645 so (layer 96 -> 32 at 256 x 256
+// 106 us, 57 GFLOP; 32 -> 32 49 us).
 __global__ void __launch_bounds__(128) k_wgrad(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap gmap,
                                                WgradParams p)
 {
@@ -236,11 +241,11 @@ __global__ void __launch_bounds__(128) k_wgrad(const __grid_constant__ CUtensorM
     const uint32_t input_row = (uint32_t)p.nc * p.row_bytes;              // one input row of a tile
     const uint32_t tile_bytes = (uint32_t)(p.ry + 2) * input_row;
     const uint32_t a_bytes = (uint32_t)p.tiles_per_cta * tile_bytes;
-    const uint32_t g_row = (uint32_t)p.tx * 16u, g_group = (uint32_t)p.ry * g_row;
+    const uint32_t g_row = p.g_row_bytes, g_group = (uint32_t)p.ry * g_row;
     const uint32_t b_bytes = (uint32_t)(p.cout / 8) * g_group;
     const uint32_t stage_bytes = a_bytes + b_bytes;
     const int g_first = t_lo * p.nc, g_count = min(nt * p.nc, p.groups - g_first);
-    const uint32_t tx_bytes = (uint32_t)(g_count * (p.ry + 2) * (p.tx + 2)) * 16u + b_bytes;
+    const uint32_t tx_bytes = (uint32_t)(g_count * (p.ry + 2) * p.tx + p.cout / 8 * p.ry * (p.tx + 2)) * 16u;
     const int S = p.stages;
     // rows past the last tile's are read (and ignored): a pad after the stages
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)S * stage_bytes + (size_t)(16 - 3 * p.nc) * p.row_bytes + 128);
@@ -248,7 +253,7 @@ __global__ void __launch_bounds__(128) k_wgrad(const __grid_constant__ CUtensorM
     uint64_t* done = empty + S;
     uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
     uint32_t* fail = tslot + 1;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31; // warp: uniform for the compiler too
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; s++) {
@@ -270,10 +275,28 @@ __global__ void __launch_bounds__(128) k_wgrad(const __grid_constant__ CUtensorM
     bool ok = true;
     const int nchunks = c_hi - c_lo;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
+        // a chunk's rows, one TMA load each, dealt out to the lanes (one thread
+        // issuing them all took 135 cycles a load); what a lane loads is the same
+        // in every chunk but for the chunk's place
+        const int n_x = g_count * (p.ry + 2), n_g = p.cout / 8 * p.ry;
+        uint32_t to[WGRAD_LANE_LOADS];
+        int channel[WGRAD_LANE_LOADS], row[WGRAD_LANE_LOADS];
+#pragma unroll
+        for (int k = 0; k < WGRAD_LANE_LOADS; k++) {
+            const int l = lane + 32 * k;
+            const bool of_x = l < n_x;
+            const int rows = of_x ? p.ry + 2 : p.ry;
+            const int g = (of_x ? l : l - n_x) / rows;
+            const int r = (of_x ? l : l - n_x) - g * rows;
+            row[k] = of_x ? r - 1 : r;
+            channel[k] = of_x ? p.x_c0 + 8 * (g_first + g) : p.g_c0 + 8 * g;
+            to[k] = of_x ? (uint32_t)(g / p.nc) * tile_bytes + (uint32_t)r * input_row + (uint32_t)(g % p.nc) * p.row_bytes
+                         : a_bytes + (uint32_t)g * g_group + (uint32_t)r * g_row;
+        }
         for (int i = 0; i < nchunks; i++) {
             const int s = i % S;
-            if (i >= S && !mbar_wait(&empty[s], (uint32_t)((i / S) - 1) & 1u)) {
+            if (!__all_sync(0xffffffffu, i < S || mbar_wait(&empty[s], (uint32_t)((i / S) - 1) & 1u))) {
                 ok = false;
                 break;
             }
@@ -284,43 +307,50 @@ __global__ void __launch_bounds__(128) k_wgrad(const __grid_constant__ CUtensorM
             const int img = c / p.chunks_y;
             const int x0 = cx * p.tx, y0 = cy * p.ry;
             uint8_t* sa = smem + (size_t)s * stage_bytes;
-            mbar_expect_tx(&full[s], tx_bytes);
-            for (int g = 0; g < g_count; g++)
-                for (int r = 0; r < p.ry + 2; r++)
-                    tma_load_4d(sa + (size_t)(g / p.nc) * tile_bytes + (size_t)r * input_row + (size_t)(g % p.nc) * p.row_bytes, &xmap,
-                                &full[s], p.x_c0 + 8 * (g_first + g), x0 - 1, y0 - 1 + r, img);
-            for (int g = 0; g < p.cout / 8; g++)
-                for (int r = 0; r < p.ry; r++)
-                    tma_load_4d(sa + a_bytes + (size_t)g * g_group + (size_t)r * g_row, &gmap, &full[s], p.g_c0 + 8 * g, x0, y0 + r, img);
+            if (lane == 0)
+                mbar_expect_tx(&full[s], tx_bytes);
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < WGRAD_LANE_LOADS; k++) {
+                const int l = lane + 32 * k;
+                if (l < n_x)
+                    tma_load_4d(sa + to[k], &xmap, &full[s], channel[k], x0, y0 + row[k], img);
+                else if (l < n_x + n_g)
+                    tma_load_4d(sa + to[k], &gmap, &full[s], channel[k], x0 - 1, y0 + row[k], img);
+            }
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
+        // the whole warp, one elected lane issuing
         const uint32_t idesc = idesc_bf16(128, (uint32_t)p.cout, true, true);
+        const uint32_t tm = __reduce_or_sync(0xffffffffu, tmem); // in a uniform register
         for (int i = 0; i < nchunks; i++) {
             const int s = i % S;
-            if (!mbar_wait(&full[s], (uint32_t)(i / S) & 1u)) {
+            if (!__all_sync(0xffffffffu, mbar_wait(&full[s], (uint32_t)(i / S) & 1u))) {
                 ok = false;
                 break;
             }
             tc_fence_after();
-            const uint32_t sa = smem_addr(smem + (size_t)s * stage_bytes);
+            const uint32_t sa = smem_addr(smem) + (uint32_t)s * stage_bytes;
             // MN-major, no swizzle: lbo = 128 between 8-pixel groups of K, sbo
             // between 8-channel groups of M/N.  A step of a descriptor's address
             // is 16 bytes: one pixel.
             uint64_t ad_y = smem_desc(sa, 128u, p.row_bytes);
-            uint64_t bd = smem_desc(sa + a_bytes, 128u, g_group);
-            for (int y = 0; y < p.ry; y++, ad_y += input_row >> 4)
-                for (int ks = 0; ks < p.tx / 16; ks++, bd += 16) {
+            uint64_t bd_y = smem_desc(sa + a_bytes, 128u, g_group);
+            for (int y = 0; y < p.ry; y++, ad_y += input_row >> 4, bd_y += g_row >> 4)
+                for (int ks = 0; ks < p.tx / 16; ks++) {
+                    const bool more = (i | y | ks) != 0;
+                    const uint64_t bd = bd_y + 16u * (uint32_t)ks;
                     uint64_t ad = ad_y + 16u * (uint32_t)ks;
-                    uint32_t d = tmem;
+                    uint32_t d = tm;
                     for (int t = 0; t < nt; t++, ad += tile_bytes >> 4, d += 3u * (uint32_t)p.cout) {
-#pragma unroll
-                        for (int kx = 0; kx < 3; kx++)
-                            mma_bf16(d + (uint32_t)(kx * p.cout), ad + kx, bd, idesc, (i | y | ks) != 0);
+                        mma_bf16_warp<FILL>(d, ad, bd + 2, idesc, more);
+                        mma_bf16_warp<USE>(d + (uint32_t)p.cout, ad, bd + 1, idesc, more);
+                        mma_bf16_warp<LAST_USE>(d + 2u * (uint32_t)p.cout, ad, bd, idesc, more);
                     }
                 }
-            mma_commit(&empty[s]);
+            mma_commit_warp(&empty[s]);
         }
-        mma_commit(done);
+        mma_commit_warp(done);
     }
     if (!ok)
         atomicOr(fail, 1u);
@@ -510,7 +540,8 @@ cudaError_t conv3x3_wgrad(const WgradCall& c, int sm_count, uint32_t* error, cud
     p.h = c.h;
     p.w = c.w;
     p.tx = wgrad_tile_width(c.w);
-    p.row_bytes = (uint32_t)(((p.tx + 2) * 16 + 127) & ~127); // TMA destinations are 128-byte aligned
+    p.row_bytes = (uint32_t)p.tx * 16; // TMA destinations are 128-byte aligned
+    p.g_row_bytes = (uint32_t)(((p.tx + 2) * 16 + 127) & ~127);
     p.dw = c.dw;
     p.error = error;
     const size_t tail = (size_t)(16 - 3 * p.nc) * p.row_bytes + 128 + 8 * (2 * 4 + 1) + 32;
@@ -518,8 +549,9 @@ cudaError_t conv3x3_wgrad(const WgradCall& c, int sm_count, uint32_t* error, cud
     // the most rows to a chunk (an input row is loaded (ry + 2) / ry times) that leave two stages, then as many
     // stages as fit
     for (p.ry = 8; p.ry >= 1; p.ry /= 2) {
-        stage = (size_t)p.tiles_per_cta * (p.ry + 2) * p.nc * p.row_bytes + (size_t)(c.cout / 8) * p.ry * p.tx * 16;
-        if ((p.ry == 1 || p.ry < 2 * c.h) && 2 * stage + tail <= SMEM_LIMIT)
+        stage = (size_t)p.tiles_per_cta * (p.ry + 2) * p.nc * p.row_bytes + (size_t)(c.cout / 8) * p.ry * p.g_row_bytes;
+        const int loads = p.tiles_per_cta * p.nc * (p.ry + 2) + c.cout / 8 * p.ry;
+        if ((p.ry == 1 || p.ry < 2 * c.h) && 2 * stage + tail <= SMEM_LIMIT && loads <= 32 * WGRAD_LANE_LOADS)
             break;
     }
     if (p.ry < 1)

@@ -69,7 +69,7 @@ bool use_rows_kernel();
 
 // dw[tap][ci][co] += sum_p x[p + offset(tap)][x_c0 + ci] * g[p][g_c0 + co]
 // over all pixels (dw must be zeroed by the caller).  x_map has a box of
-// wgrad_tile_width + 2 pixels of one row, g_map one of wgrad_tile_width.
+// wgrad_tile_width pixels of one row, g_map one of wgrad_tile_width + 2.
 struct WgradCall {
     const CUtensorMap* x_map;
     int x_c0, cin;

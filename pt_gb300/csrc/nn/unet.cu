@@ -127,7 +127,7 @@ bool UNet::make(Buf& b, int level, int channels, std::string& err)
         return false;
     }
     tx = wgrad_tile_width(b.a.w);
-    if (!encode_act_map(&b.wg_x, b.a, tx + 2, 1, &why) || !encode_act_map(&b.wg_g, b.a, tx, 1, &why)) {
+    if (!encode_act_map(&b.wg_x, b.a, tx, 1, &why) || !encode_act_map(&b.wg_g, b.a, tx + 2, 1, &why)) {
         err = why;
         return false;
     }
