@@ -1,25 +1,19 @@
 // ops.cu — memory-bound kernels of the denoiser: 2x2 average pooling and
 // nearest upsampling with their backward passes (ReLU masks fused), bias
-// gradients, weight packing for the tensor-core layouts and Adam.  Each
-// thread moves 8 channels (one 16-byte vector) of one pixel.
+// gradients, weight packing for the tensor-core layouts and Adam.  A thread of
+// the pooling and upsampling kernels moves 16 channels (32-byte accesses) of
+// one low-resolution pixel and its four high-resolution ones.
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include "nn.h"
+#include "tc.cuh"
 
 namespace pt {
 namespace nn {
 
 namespace {
-
-__device__ __forceinline__ void unpack8(uint4 q, float (&v)[8])
-{
-    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        v[2 * k] = __uint_as_float(w[k] << 16);
-        v[2 * k + 1] = __uint_as_float(w[k] & 0xFFFF0000u);
-    }
-}
 
 __device__ __forceinline__ uint32_t pack2(float a, float b)
 {
@@ -27,155 +21,193 @@ __device__ __forceinline__ uint32_t pack2(float a, float b)
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
-__device__ __forceinline__ uint4 pack8(const float (&v)[8])
-{
-    return make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
-}
-
-__device__ __forceinline__ uint4 ld8(const Act& a, size_t pix, int c)
-{
-    return *reinterpret_cast<const uint4*>(a.p + pix * a.pitch + c);
-}
-
-__device__ __forceinline__ void st8(const Act& a, size_t pix, int c, uint4 v)
-{
-    *reinterpret_cast<uint4*>(a.p + pix * a.pitch + c) = v;
-}
-
 __device__ __forceinline__ size_t pixel(const Act& a, int img, int y, int x)
 {
     return ((size_t)img * a.h + y) * a.w + x;
 }
 
-// grid-stride over (output pixel, 8-channel group)
-#define PT_FOR_PIXEL_GROUPS(out, groups)                                                                                          \
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x, n_ = (out).pixels() * (groups); i < n_;                       \
-         i += (size_t)gridDim.x * blockDim.x)
+// 16 channels from c of a pixel, as floats or as they are.
+struct Vec16 {
+    uint32_t w[8];
+    __device__ __forceinline__ float lo(int k) const { return __uint_as_float(w[k] << 16); }
+    __device__ __forceinline__ float hi(int k) const { return __uint_as_float(w[k] & 0xFFFF0000u); }
+};
 
-__global__ void k_pool2(Act in, int in_c0, int groups, Act out, int out_c0)
+__device__ __forceinline__ Vec16 ld16(const Act& a, size_t pix, int c)
 {
-    PT_FOR_PIXEL_GROUPS(out, groups)
-    {
-        const int g = (int)(i % groups);
-        size_t q = i / groups;
-        const int x = (int)(q % out.w);
-        q /= out.w;
-        const int y = (int)(q % out.h);
-        const int img = (int)(q / out.h);
-        float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int dy = 0; dy < 2; dy++)
-            for (int dx = 0; dx < 2; dx++) {
-                float v[8];
-                unpack8(ld8(in, pixel(in, img, 2 * y + dy, 2 * x + dx), in_c0 + 8 * g), v);
-#pragma unroll
-                for (int k = 0; k < 8; k++)
-                    acc[k] += v[k];
-            }
-#pragma unroll
-        for (int k = 0; k < 8; k++)
-            acc[k] *= 0.25f;
-        st8(out, pixel(out, img, y, x), out_c0 + 8 * g, pack8(acc));
-    }
+    Vec16 v;
+    load32(a.p + pix * a.pitch + c, v.w);
+    return v;
 }
 
-__global__ void k_upsample2(Act in, int in_c0, int groups, Act out, int out_c0)
-{
-    PT_FOR_PIXEL_GROUPS(out, groups)
-    {
-        const int g = (int)(i % groups);
-        size_t q = i / groups;
-        const int x = (int)(q % out.w);
-        q /= out.w;
-        const int y = (int)(q % out.h);
-        const int img = (int)(q / out.h);
-        st8(out, pixel(out, img, y, x), out_c0 + 8 * g, ld8(in, pixel(in, img, y / 2, x / 2), in_c0 + 8 * g));
-    }
-}
+__device__ __forceinline__ void st16(const Act& a, size_t pix, int c, const Vec16& v) { store32(a.p + pix * a.pitch + c, v.w); }
 
-__device__ __forceinline__ void relu_mask(float (&v)[8], uint4 zq)
+__device__ __forceinline__ Vec16 pack16(const float (&v)[16])
 {
-    float z[8];
-    unpack8(zq, z);
+    Vec16 r;
 #pragma unroll
     for (int k = 0; k < 8; k++)
-        if (!(z[k] > 0.0f))
-            v[k] = 0.0f;
+        r.w[k] = pack2(v[2 * k], v[2 * k + 1]);
+    return r;
 }
 
-__global__ void k_upsample2_backward(Act gh, int g_c0, int groups, Act z, int z_c0, Act gl)
+__device__ __forceinline__ void add16(float (&acc)[16], const Vec16& v)
 {
-    PT_FOR_PIXEL_GROUPS(gl, groups)
-    {
-        const int g = (int)(i % groups);
-        size_t q = i / groups;
-        const int x = (int)(q % gl.w);
-        q /= gl.w;
-        const int y = (int)(q % gl.h);
-        const int img = (int)(q / gl.h);
-        float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int dy = 0; dy < 2; dy++)
-            for (int dx = 0; dx < 2; dx++) {
-                float v[8];
-                unpack8(ld8(gh, pixel(gh, img, 2 * y + dy, 2 * x + dx), g_c0 + 8 * g), v);
 #pragma unroll
-                for (int k = 0; k < 8; k++)
-                    acc[k] += v[k];
-            }
-        const size_t pl = pixel(gl, img, y, x);
-        relu_mask(acc, ld8(z, pl, z_c0 + 8 * g));
-        st8(gl, pl, 8 * g, pack8(acc));
+    for (int k = 0; k < 8; k++) {
+        acc[2 * k] += v.lo(k);
+        acc[2 * k + 1] += v.hi(k);
     }
 }
 
-__global__ void k_pool2_backward(Act gs, int s_c0, Act gp, int groups, Act z, int z_c0, Act g_out)
+// Zeroes the channels whose activation z is not positive.
+__device__ __forceinline__ void relu_mask(float (&v)[16], const Vec16& z)
 {
-    PT_FOR_PIXEL_GROUPS(g_out, groups)
-    {
-        const int g = (int)(i % groups);
-        size_t q = i / groups;
-        const int x = (int)(q % g_out.w);
-        q /= g_out.w;
-        const int y = (int)(q % g_out.h);
-        const int img = (int)(q / g_out.h);
-        const size_t ph = pixel(g_out, img, y, x);
-        float a[8], b[8];
-        unpack8(ld8(gs, ph, s_c0 + 8 * g), a);
-        unpack8(ld8(gp, pixel(gp, img, y / 2, x / 2), 8 * g), b);
 #pragma unroll
-        for (int k = 0; k < 8; k++)
-            a[k] += 0.25f * b[k];
-        relu_mask(a, ld8(z, ph, z_c0 + 8 * g));
-        st8(g_out, ph, 8 * g, pack8(a));
+    for (int k = 0; k < 8; k++) {
+        if (!(z.lo(k) > 0.0f))
+            v[2 * k] = 0.0f;
+        if (!(z.hi(k) > 0.0f))
+            v[2 * k + 1] = 0.0f;
     }
 }
 
-// One block reduces a pixel range for all channels: thread t owns the 8-channel
-// group t % groups and strides over pixels by blockDim / groups.
-__global__ void k_bias_grad(Act g, int c0, int groups, float* db, size_t pixels_per_block)
+// f(img, y, x, u): every pixel of `low` and unit u of `units` units of 16
+// channels.  Rows over blockIdx.y, so that one 32-bit division finds the pixel.
+// With 64-bit divisions of a flat index and 16-byte accesses upsampling was bound
+// by its integer arithmetic (64 channels to 1080 x 1920, 331 MB: 81 us, 50 now;
+// backward at 16 x 256 x 256: 39 us, 25 now).  Pooling is bound by DRAM before
+// and after (42 us at 6.6 TB/s): the skip connection is 64 bytes of a pixel's 192
+// and DRAM delivers 128.
+template <class F>
+__device__ __forceinline__ void for_low_pixels(const Act& low, int units, F f)
 {
-    extern __shared__ float red[];
-    const int rows = blockDim.x / groups;
-    const int grp = threadIdx.x % groups, row = threadIdx.x / groups;
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    const size_t p0 = blockIdx.x * pixels_per_block;
-    const size_t p1 = min(p0 + pixels_per_block, g.pixels());
-    if (row < rows)
-        for (size_t p = p0 + row; p < p1; p += rows) {
-            float v[8];
-            unpack8(ld8(g, p, c0 + 8 * grp), v);
-#pragma unroll
-            for (int k = 0; k < 8; k++)
-                acc[k] += v[k];
+    const uint32_t rows = (uint32_t)low.n * (uint32_t)low.h, row_units = (uint32_t)low.w * (uint32_t)units;
+    for (uint32_t row = blockIdx.y; row < rows; row += gridDim.y) {
+        const uint32_t img = row / (uint32_t)low.h, y = row - img * (uint32_t)low.h;
+        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < row_units; i += gridDim.x * blockDim.x) {
+            const uint32_t x = i / (uint32_t)units;
+            f((int)img, (int)y, (int)x, (int)(i - x * (uint32_t)units));
         }
-    for (int k = 0; k < 8; k++)
-        red[threadIdx.x * 8 + k] = row < rows ? acc[k] : 0.0f;
+    }
+}
+
+constexpr int POOL_THREADS = 128;
+
+__global__ void __launch_bounds__(POOL_THREADS) k_pool2(Act in, int in_c0, int units, Act out, int out_c0)
+{
+    for_low_pixels(out, units, [&](int img, int y, int x, int u) {
+        float acc[16] = {};
+        const size_t p = pixel(in, img, 2 * y, 2 * x);
+        const Vec16 v00 = ld16(in, p, in_c0 + 16 * u), v01 = ld16(in, p + 1, in_c0 + 16 * u);
+        const Vec16 v10 = ld16(in, p + in.w, in_c0 + 16 * u), v11 = ld16(in, p + in.w + 1, in_c0 + 16 * u);
+        add16(acc, v00);
+        add16(acc, v01);
+        add16(acc, v10);
+        add16(acc, v11);
+#pragma unroll
+        for (int k = 0; k < 16; k++)
+            acc[k] *= 0.25f;
+        st16(out, pixel(out, img, y, x), out_c0 + 16 * u, pack16(acc));
+    });
+}
+
+__global__ void __launch_bounds__(POOL_THREADS) k_upsample2(Act in, int in_c0, int units, Act out, int out_c0)
+{
+    for_low_pixels(in, units, [&](int img, int y, int x, int u) {
+        const Vec16 v = ld16(in, pixel(in, img, y, x), in_c0 + 16 * u);
+        const size_t p = pixel(out, img, 2 * y, 2 * x);
+        const int c = out_c0 + 16 * u;
+        st16(out, p, c, v);
+        st16(out, p + 1, c, v);
+        st16(out, p + out.w, c, v);
+        st16(out, p + out.w + 1, c, v);
+    });
+}
+
+__global__ void __launch_bounds__(POOL_THREADS) k_upsample2_backward(Act gh, int g_c0, int units, Act z, int z_c0, Act gl)
+{
+    for_low_pixels(gl, units, [&](int img, int y, int x, int u) {
+        float acc[16] = {};
+        const size_t p = pixel(gh, img, 2 * y, 2 * x), pl = pixel(gl, img, y, x);
+        const int c = g_c0 + 16 * u;
+        const Vec16 v00 = ld16(gh, p, c), v01 = ld16(gh, p + 1, c), v10 = ld16(gh, p + gh.w, c), v11 = ld16(gh, p + gh.w + 1, c);
+        const Vec16 zv = ld16(z, pl, z_c0 + 16 * u);
+        add16(acc, v00);
+        add16(acc, v01);
+        add16(acc, v10);
+        add16(acc, v11);
+        relu_mask(acc, zv);
+        st16(gl, pl, 16 * u, pack16(acc));
+    });
+}
+
+__global__ void __launch_bounds__(POOL_THREADS) k_pool2_backward(Act gs, int s_c0, Act gp, int units, Act z, int z_c0, Act g_out)
+{
+    for_low_pixels(gp, units, [&](int img, int y, int x, int u) {
+        const Vec16 b = ld16(gp, pixel(gp, img, y, x), 16 * u);
+        const size_t p0 = pixel(g_out, img, 2 * y, 2 * x);
+        // a pixel at a time: all eight loads first is slower (21 -> 23 us a level
+        // below), for the registers cost more warps than the loads ahead give
+#pragma unroll
+        for (int d = 0; d < 4; d++) {
+            const size_t p = p0 + (size_t)(d >> 1) * g_out.w + (d & 1);
+            const Vec16 s = ld16(gs, p, s_c0 + 16 * u), zv = ld16(z, p, z_c0 + 16 * u);
+            float a[16];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                a[2 * k] = s.lo(k) + 0.25f * b.lo(k);
+                a[2 * k + 1] = s.hi(k) + 0.25f * b.hi(k);
+            }
+            relu_mask(a, zv);
+            st16(g_out, p, 16 * u, pack16(a));
+        }
+    });
+}
+
+// One block reduces a pixel range for all channels: thread t owns the 16-channel
+// unit t % units and strides over pixels by the block's rows, four 32-byte loads
+// ahead of the sums: 32 channels of 16 x 256 x 256 (67 MB) take 14 us, 19 with one
+// 16-byte load at a time.
+constexpr int BIAS_THREADS = 256;
+
+__global__ void __launch_bounds__(BIAS_THREADS) k_bias_grad(Act g, int c0, int units, float* db, uint32_t pixels_per_block)
+{
+    __shared__ float red[BIAS_THREADS * 17];
+    const int rows = BIAS_THREADS / units;
+    const int u = threadIdx.x % units, row = threadIdx.x / units;
+    float acc[16] = {};
+    const size_t p0 = blockIdx.x * (size_t)pixels_per_block;
+    const size_t left = g.pixels() - p0;
+    const int n = (int)(left < pixels_per_block ? left : pixels_per_block);
+    if (row < rows) {
+        const uint16_t* q = g.p + p0 * g.pitch + c0 + 16 * u;
+        int p = row;
+        for (; p + 3 * rows < n; p += 4 * rows) {
+            Vec16 v[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                load32(q + (size_t)(p + k * rows) * g.pitch, v[k].w);
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                add16(acc, v[k]);
+        }
+        for (; p < n; p += rows) {
+            Vec16 v;
+            load32(q + (size_t)p * g.pitch, v.w);
+            add16(acc, v);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 16; k++)
+        red[threadIdx.x * 17 + k] = acc[k];
     __syncthreads();
-    if (threadIdx.x < groups * 8) {
-        const int gg = threadIdx.x / 8, k = threadIdx.x % 8;
+    if ((int)threadIdx.x < units * 16) {
+        const int uu = threadIdx.x / 16, k = threadIdx.x % 16;
         float s = 0.0f;
         for (int r = 0; r < rows; r++)
-            s += red[(r * groups + gg) * 8 + k];
-        atomicAdd(db + 8 * gg + k, s);
+            s += red[(r * units + uu) * 17 + k];
+        atomicAdd(db + 16 * uu + k, s);
     }
 }
 
@@ -222,57 +254,67 @@ bool shape_ok(const Act& a, int c0, int c)
     return a.p && c > 0 && c % 8 == 0 && c0 % 8 == 0 && c0 + c <= a.pitch && a.pitch % 8 == 0;
 }
 
+// ... and for the kernels with 32-byte accesses.
+bool shape_ok16(const Act& a, int c0, int c)
+{
+    return shape_ok(a, c0, c) && c % 16 == 0 && c0 % 16 == 0 && a.pitch % 16 == 0 && ((uintptr_t)a.p & 31) == 0;
+}
+
+dim3 low_grid(const Act& low, int units)
+{
+    const unsigned x = (unsigned)(((uint64_t)low.w * units + POOL_THREADS - 1) / POOL_THREADS);
+    return dim3(x, (unsigned)std::min<uint64_t>((uint64_t)low.n * low.h, 65535));
+}
+
 } // namespace
 
 cudaError_t pool2(const Act& in, int in_c0, int c, const Act& out, int out_c0, cudaStream_t st)
 {
-    if (!shape_ok(in, in_c0, c) || !shape_ok(out, out_c0, c) || in.h != 2 * out.h || in.w != 2 * out.w || in.n != out.n)
+    if (!shape_ok16(in, in_c0, c) || !shape_ok16(out, out_c0, c) || in.h != 2 * out.h || in.w != 2 * out.w || in.n != out.n)
         return cudaErrorInvalidValue;
-    k_pool2<<<grid_for(out.pixels() * (c / 8), 256), 256, 0, st>>>(in, in_c0, c / 8, out, out_c0);
+    k_pool2<<<low_grid(out, c / 16), POOL_THREADS, 0, st>>>(in, in_c0, c / 16, out, out_c0);
     return cudaGetLastError();
 }
 
 cudaError_t upsample2(const Act& in, int in_c0, int c, const Act& out, int out_c0, cudaStream_t st)
 {
-    if (!shape_ok(in, in_c0, c) || !shape_ok(out, out_c0, c) || out.h != 2 * in.h || out.w != 2 * in.w || in.n != out.n)
+    if (!shape_ok16(in, in_c0, c) || !shape_ok16(out, out_c0, c) || out.h != 2 * in.h || out.w != 2 * in.w || in.n != out.n)
         return cudaErrorInvalidValue;
-    k_upsample2<<<grid_for(out.pixels() * (c / 8), 256), 256, 0, st>>>(in, in_c0, c / 8, out, out_c0);
+    k_upsample2<<<low_grid(in, c / 16), POOL_THREADS, 0, st>>>(in, in_c0, c / 16, out, out_c0);
     return cudaGetLastError();
 }
 
 cudaError_t upsample2_backward(const Act& g_high, int g_c0, int c, const Act& z, int z_c0, const Act& g_low, cudaStream_t st)
 {
-    if (!shape_ok(g_high, g_c0, c) || !shape_ok(z, z_c0, c) || !shape_ok(g_low, 0, c) || g_high.h != 2 * g_low.h ||
+    if (!shape_ok16(g_high, g_c0, c) || !shape_ok16(z, z_c0, c) || !shape_ok16(g_low, 0, c) || g_high.h != 2 * g_low.h ||
         g_high.w != 2 * g_low.w || z.h != g_low.h || z.w != g_low.w)
         return cudaErrorInvalidValue;
-    k_upsample2_backward<<<grid_for(g_low.pixels() * (c / 8), 256), 256, 0, st>>>(g_high, g_c0, c / 8, z, z_c0, g_low);
+    k_upsample2_backward<<<low_grid(g_low, c / 16), POOL_THREADS, 0, st>>>(g_high, g_c0, c / 16, z, z_c0, g_low);
     return cudaGetLastError();
 }
 
 cudaError_t pool2_backward(const Act& g_skip, int s_c0, const Act& g_pool, int c, const Act& z, int z_c0, const Act& g,
                            cudaStream_t st)
 {
-    if (!shape_ok(g_skip, s_c0, c) || !shape_ok(g_pool, 0, c) || !shape_ok(z, z_c0, c) || !shape_ok(g, 0, c) ||
+    if (!shape_ok16(g_skip, s_c0, c) || !shape_ok16(g_pool, 0, c) || !shape_ok16(z, z_c0, c) || !shape_ok16(g, 0, c) ||
         g.h != 2 * g_pool.h || g.w != 2 * g_pool.w || g_skip.h != g.h || z.h != g.h)
         return cudaErrorInvalidValue;
-    k_pool2_backward<<<grid_for(g.pixels() * (c / 8), 256), 256, 0, st>>>(g_skip, s_c0, g_pool, c / 8, z, z_c0, g);
+    k_pool2_backward<<<low_grid(g_pool, c / 16), POOL_THREADS, 0, st>>>(g_skip, s_c0, g_pool, c / 16, z, z_c0, g);
     return cudaGetLastError();
 }
 
 cudaError_t bias_grad(const Act& g, int c0, int c, float* db, cudaStream_t st)
 {
-    if (!shape_ok(g, c0, c) || c > 256)
+    if (!shape_ok16(g, c0, c) || c > BIAS_THREADS)
         return cudaErrorInvalidValue;
-    const int groups = c / 8;
-    const int threads = 256;
+    // four blocks per SM, and no block below 128 pixels: its reduction costs as much
     const size_t blocks = 152 * 4;
     size_t per = (g.pixels() + blocks - 1) / blocks;
-    if (per == 0)
-        per = 1;
+    per = std::max<size_t>(per, 128);
     const size_t nb = (g.pixels() + per - 1) / per;
     if (nb == 0)
         return cudaSuccess;
-    k_bias_grad<<<(unsigned)nb, threads, threads * 8 * sizeof(float), st>>>(g, c0, groups, db, per);
+    k_bias_grad<<<(unsigned)nb, BIAS_THREADS, 0, st>>>(g, c0, c / 16, db, (uint32_t)per);
     return cudaGetLastError();
 }
 

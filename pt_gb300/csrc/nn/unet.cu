@@ -47,7 +47,9 @@ size_t param_count()
 
 namespace {
 
-__global__ void k_loss(const float* out32, const float4* target, size_t pixels, uint16_t* g_out, double* loss_acc)
+constexpr int LOSS_THREADS = 256;
+
+__global__ void __launch_bounds__(LOSS_THREADS) k_loss(const float* out32, const float4* target, size_t pixels, uint16_t* g_out, double* loss_acc)
 {
     double local = 0.0;
     const float scale = 2.0f / (3.0f * (float)pixels);
@@ -72,8 +74,16 @@ __global__ void k_loss(const float* out32, const float4* target, size_t pixels, 
     }
     for (int o = 16; o > 0; o >>= 1)
         local += __shfl_down_sync(0xffffffffu, local, o);
+    // one atomic a block: all of them go to one address
+    __shared__ double warp_sum[LOSS_THREADS / 32];
     if ((threadIdx.x & 31) == 0)
+        warp_sum[threadIdx.x / 32] = local;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < LOSS_THREADS / 32; i++)
+            local += warp_sum[i];
         atomicAdd(loss_acc, local);
+    }
 }
 
 } // namespace
@@ -81,10 +91,10 @@ __global__ void k_loss(const float* out32, const float4* target, size_t pixels, 
 cudaError_t loss_backward(const float* out32, const float* target, size_t pixels, uint16_t* g_out, double* loss_acc,
                           cudaStream_t st)
 {
-    size_t blocks = (pixels + 255) / 256;
+    size_t blocks = (pixels + LOSS_THREADS - 1) / LOSS_THREADS;
     if (blocks > 152 * 8)
         blocks = 152 * 8;
-    k_loss<<<(unsigned)(blocks ? blocks : 1), 256, 0, st>>>(out32, reinterpret_cast<const float4*>(target), pixels, g_out,
+    k_loss<<<(unsigned)(blocks ? blocks : 1), LOSS_THREADS, 0, st>>>(out32, reinterpret_cast<const float4*>(target), pixels, g_out,
                                                              loss_acc);
     return cudaGetLastError();
 }
