@@ -18,6 +18,7 @@
 
 #include <algorithm>
 
+#include "../device/chain.cuh"
 #include "nn.h"
 #include "tc.cuh"
 
@@ -56,6 +57,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b)
 
 __global__ void __launch_bounds__(128) k_conv3x3(const __grid_constant__ CUtensorMap amap, ConvParams p)
 {
+    chain_begin();
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t a_bytes = (uint32_t)p.cin * 256u;
     const uint32_t b_bytes = (uint32_t)p.nout * (uint32_t)p.cin * 2u;
@@ -232,6 +234,7 @@ struct WgradParams {
 __global__ void __launch_bounds__(128) k_wgrad(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap gmap,
                                                WgradParams p)
 {
+    chain_begin();
     extern __shared__ __align__(1024) uint8_t smem[];
     const int t_lo = blockIdx.x * p.tiles_per_cta, nt = min(p.tiles_per_cta, p.tiles - t_lo);
     const int c_lo = blockIdx.y * p.chunks_per_cta;
@@ -519,7 +522,7 @@ cudaError_t conv3x3(const ConvCall& c, uint32_t* error, cudaStream_t st)
     const long long tiles = (long long)p.tiles_x * p.tiles_y * p.n;
     if (tiles <= 0)
         return cudaSuccess;
-    k_conv3x3<<<(unsigned)tiles, 128, smem, st>>>(*c.in_map, p);
+    launch_chained(k_conv3x3, (unsigned)tiles, 128, smem, st, *c.in_map, p);
     return cudaGetLastError();
 }
 
@@ -572,7 +575,7 @@ cudaError_t conv3x3_wgrad(const WgradCall& c, int sm_count, uint32_t* error, cud
     cudaError_t e = cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_LIMIT);
     if (e != cudaSuccess)
         return e;
-    k_wgrad<<<dim3((unsigned)cta_x, (unsigned)splits), 128, smem, st>>>(*c.x_map, *c.g_map, p);
+    launch_chained(k_wgrad, dim3((unsigned)cta_x, (unsigned)splits), 128, smem, st, *c.x_map, *c.g_map, p);
     return cudaGetLastError();
 }
 

@@ -28,6 +28,7 @@
 #include <algorithm>
 #include <cstdlib>
 
+#include "../device/chain.cuh"
 #include "nn.h"
 #include "tc.cuh"
 
@@ -182,6 +183,7 @@ __device__ __forceinline__ void input_row(uint32_t d, uint64_t ad, uint64_t bd, 
 
 __global__ void __launch_bounds__(ROWS_THREADS) k_conv3x3_rows(const __grid_constant__ CUtensorMap amap, RowsParams p)
 {
+    chain_begin();
     extern __shared__ __align__(1024) uint8_t smem[];
     const int MT = p.mt;
     // one 8-channel halo, rounded up so every TMA destination is 128-byte aligned
@@ -355,6 +357,7 @@ __global__ void __launch_bounds__(ROWS_THREADS) k_conv3x3_rows(const __grid_cons
 
 __global__ void k_pack_rows(const float* w, int cin, int cout, uint16_t* fwd, uint16_t* bwd)
 {
+    chain_begin();
     const size_t n = (size_t)9 * cin * cout;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const int co = (int)(i % cout);
@@ -462,7 +465,7 @@ cudaError_t conv3x3_rows(const ConvCall& c, const CUtensorMap* halo_map, int sm_
     }
     // one CTA per SM (its two accumulator buffers may take all 512 TMEM columns)
     const int grid = std::min(p.tiles, sm_count);
-    k_conv3x3_rows<<<grid, ROWS_THREADS, smem, st>>>(*halo_map, p);
+    launch_chained(k_conv3x3_rows, grid, ROWS_THREADS, smem, st, *halo_map, p);
     return cudaGetLastError();
 }
 

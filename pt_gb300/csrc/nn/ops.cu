@@ -7,6 +7,7 @@
 
 #include <algorithm>
 
+#include "../device/chain.cuh"
 #include "nn.h"
 #include "tc.cuh"
 
@@ -96,6 +97,7 @@ constexpr int POOL_THREADS = 128;
 
 __global__ void __launch_bounds__(POOL_THREADS) k_pool2(Act in, int in_c0, int units, Act out, int out_c0)
 {
+    chain_begin();
     for_low_pixels(out, units, [&](int img, int y, int x, int u) {
         float acc[16] = {};
         const size_t p = pixel(in, img, 2 * y, 2 * x);
@@ -114,6 +116,7 @@ __global__ void __launch_bounds__(POOL_THREADS) k_pool2(Act in, int in_c0, int u
 
 __global__ void __launch_bounds__(POOL_THREADS) k_upsample2(Act in, int in_c0, int units, Act out, int out_c0)
 {
+    chain_begin();
     for_low_pixels(in, units, [&](int img, int y, int x, int u) {
         const Vec16 v = ld16(in, pixel(in, img, y, x), in_c0 + 16 * u);
         const size_t p = pixel(out, img, 2 * y, 2 * x);
@@ -127,6 +130,7 @@ __global__ void __launch_bounds__(POOL_THREADS) k_upsample2(Act in, int in_c0, i
 
 __global__ void __launch_bounds__(POOL_THREADS) k_upsample2_backward(Act gh, int g_c0, int units, Act z, int z_c0, Act gl)
 {
+    chain_begin();
     for_low_pixels(gl, units, [&](int img, int y, int x, int u) {
         float acc[16] = {};
         const size_t p = pixel(gh, img, 2 * y, 2 * x), pl = pixel(gl, img, y, x);
@@ -144,6 +148,7 @@ __global__ void __launch_bounds__(POOL_THREADS) k_upsample2_backward(Act gh, int
 
 __global__ void __launch_bounds__(POOL_THREADS) k_pool2_backward(Act gs, int s_c0, Act gp, int units, Act z, int z_c0, Act g_out)
 {
+    chain_begin();
     for_low_pixels(gp, units, [&](int img, int y, int x, int u) {
         const Vec16 b = ld16(gp, pixel(gp, img, y, x), 16 * u);
         const size_t p0 = pixel(g_out, img, 2 * y, 2 * x);
@@ -173,6 +178,7 @@ constexpr int BIAS_THREADS = 256;
 
 __global__ void __launch_bounds__(BIAS_THREADS) k_bias_grad(Act g, int c0, int units, float* db, uint32_t pixels_per_block)
 {
+    chain_begin();
     __shared__ float red[BIAS_THREADS * 17];
     const int rows = BIAS_THREADS / units;
     const int u = threadIdx.x % units, row = threadIdx.x / units;
@@ -314,7 +320,7 @@ cudaError_t bias_grad(const Act& g, int c0, int c, float* db, cudaStream_t st)
     const size_t nb = (g.pixels() + per - 1) / per;
     if (nb == 0)
         return cudaSuccess;
-    k_bias_grad<<<(unsigned)nb, BIAS_THREADS, 0, st>>>(g, c0, c / 16, db, (uint32_t)per);
+    launch_chained(k_bias_grad, (unsigned)nb, BIAS_THREADS, 0, st, g, c0, c / 16, db, (uint32_t)per);
     return cudaGetLastError();
 }
 

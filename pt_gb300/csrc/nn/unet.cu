@@ -16,6 +16,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "../device/chain.cuh"
 #include "unet.h"
 
 namespace pt {
@@ -51,6 +52,7 @@ constexpr int LOSS_THREADS = 256;
 
 __global__ void __launch_bounds__(LOSS_THREADS) k_loss(const float* out32, const float4* target, size_t pixels, uint16_t* g_out, double* loss_acc)
 {
+    chain_begin();
     double local = 0.0;
     const float scale = 2.0f / (3.0f * (float)pixels);
     for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < pixels; p += (size_t)gridDim.x * blockDim.x) {
@@ -94,8 +96,7 @@ cudaError_t loss_backward(const float* out32, const float* target, size_t pixels
     size_t blocks = (pixels + LOSS_THREADS - 1) / LOSS_THREADS;
     if (blocks > 152 * 8)
         blocks = 152 * 8;
-    k_loss<<<(unsigned)(blocks ? blocks : 1), LOSS_THREADS, 0, st>>>(out32, reinterpret_cast<const float4*>(target), pixels, g_out,
-                                                             loss_acc);
+    k_loss<<<(unsigned)(blocks ? blocks : 1), LOSS_THREADS, 0, st>>>(out32, reinterpret_cast<const float4*>(target), pixels, g_out, loss_acc);
     return cudaGetLastError();
 }
 

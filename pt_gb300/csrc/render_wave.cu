@@ -38,6 +38,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "device/chain.cuh"
 #include "device/order.h"
 #include "device/render.cuh"
 #include "kernels.h"
@@ -414,6 +415,7 @@ __global__ void __launch_bounds__(128, 8) k_wf_extend_resume(WaveArgs<Src> a)
 template <class Src>
 __global__ void __launch_bounds__(256) k_wf_split(WaveArgs<Src> a, uint32_t qi)
 {
+    chain_begin();
     __shared__ uint32_t s_warp[8];
     __shared__ uint32_t s_base;
     const uint32_t* queue = a.w.queue[qi];
@@ -497,6 +499,7 @@ struct NeeToWave {
 template <class Src, int MINB, bool PLAIN>
 __global__ void __launch_bounds__(128, MINB) k_wf_shade(WaveArgs<Src> a, uint32_t qi)
 {
+    chain_begin();
     const uint32_t* qin = a.w.hit_queue;
     uint32_t* qout = a.w.queue[qi ^ 1];
     const uint32_t count = *hit_count(a.w.counts, qi);
@@ -657,6 +660,7 @@ __device__ __forceinline__ void finish_shadow_entry(WaveArgs<Src>& a, uint32_t p
 template <class Src, bool W4>
 __global__ void __launch_bounds__(128) k_wf_shadow_refill(WaveArgs<Src> a, uint32_t refill)
 {
+    chain_begin();
     const uint32_t count = a.w.counts[2];
     const unsigned lane = threadIdx.x & 31;
     const unsigned lower = (1u << lane) - 1u;
@@ -731,6 +735,7 @@ __device__ __forceinline__ void shadow_finish(const WaveArgs<Src>& a, uint32_t p
 template <class Src, bool W4, bool BUDGET = false>
 __global__ void __launch_bounds__(128, W4 ? 8 : 1) k_wf_shadow(WaveArgs<Src> a, uint32_t budget)
 {
+    chain_begin();
     const uint32_t count = a.w.counts[2];
     unsigned lane = threadIdx.x & 31;
     const uint32_t take = rays_per_fetch(count);
@@ -792,6 +797,7 @@ __global__ void __launch_bounds__(128, W4 ? 8 : 1) k_wf_shadow(WaveArgs<Src> a, 
 template <class Src>
 __global__ void __launch_bounds__(128, 7) k_wf_shadow_resume(WaveArgs<Src> a)
 {
+    chain_begin();
     const uint32_t parked = *(volatile uint32_t*)&a.w.counts[8];
     const uint32_t count = parked < a.w.park.cap ? parked : a.w.park.cap;
     const unsigned lane = threadIdx.x & 31;
@@ -835,6 +841,7 @@ __global__ void __launch_bounds__(128, 7) k_wf_shadow_resume(WaveArgs<Src> a)
 // traversal's in split, the path queue's and the other hit queue's in shade.
 __global__ void k_wf_reset(uint32_t* counts)
 {
+    chain_begin();
     counts[2] = 0;
     counts[4] = 0;
     counts[8] = 0;
@@ -1114,11 +1121,11 @@ template <class Src, bool PLAIN>
 static void launch_shade(int resident, uint32_t grid, cudaStream_t st, const WaveArgs<Src>& a, uint32_t qi)
 {
     if (resident == 5)
-        k_wf_shade<Src, 5, PLAIN><<<grid, 128, 0, st>>>(a, qi);
+        launch_chained(k_wf_shade<Src, 5, PLAIN>, grid, 128, 0, st, a, qi);
     else if (resident == 6)
-        k_wf_shade<Src, 6, PLAIN><<<grid, 128, 0, st>>>(a, qi);
+        launch_chained(k_wf_shade<Src, 6, PLAIN>, grid, 128, 0, st, a, qi);
     else
-        k_wf_shade<Src, 0, PLAIN><<<grid, 128, 0, st>>>(a, qi);
+        launch_chained(k_wf_shade<Src, 0, PLAIN>, grid, 128, 0, st, a, qi);
 }
 
 // One wave: raygen, (extend, shade, shadow, reset) per segment, accumulate.
@@ -1196,7 +1203,7 @@ static uint32_t launch_wave(const WaveArgs<Src>& a, bool w4, bool plain, uint32_
         else
             k_wf_shadow<Src, false><<<shadow_blocks, 128, 0, sst>>>(a, 0u);
         mark(4);
-        k_wf_reset<<<1, 1, 0, sst>>>(a.w.counts);
+        launch_chained(k_wf_reset, 1, 1, 0, sst, a.w.counts);
         if (overlap)
             cudaEventRecord(shadow.traced, sst);
         nl += 5;
