@@ -28,6 +28,7 @@
 // run until every segment is small; then one block per segment finishes it in
 // shared memory.  Nodes are numbered in merge order by prefix sums
 // (deterministic).  PT_BVH=lbvh selects the radix tree instead (kept for A/B).
+#include <cooperative_groups.h>
 #include <cub/cub.cuh>
 #include <thrust/iterator/counting_iterator.h>
 #include <thrust/iterator/transform_iterator.h>
@@ -41,6 +42,8 @@
 #include "kernels.h"
 
 namespace pt {
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -649,8 +652,15 @@ __global__ void k_ploc_init(Scratch s, uint32_t n, int mode_tlas)
 // clusters k0 .. k1 + 1 (k0, k1 even) staged in shared memory, `stride` floats
 // each of lo.x, lo.y, lo.z, hi.x, hi.y, hi.z: of those at most `radius` away (and
 // of the own segment, SEG; below n otherwise) the one whose box merges with the
-// smallest surface, of equal ones the first (the lower index pair).  Two boxes
-// are read at a time, four distances per six 8-byte reads.
+// smallest surface, of equal ones the first (the lower index pair).
+//
+// Inside the window (all but its ends and the pair itself) nothing needs testing
+// when both of its ends belong to the pair's segment: clusters are in their
+// segments' order.  There four clusters are read at a time and only the smallest
+// of their four distances is compared; which of the four it was is found at the
+// end.  The kernels that call it are bound by the ALU pipe (minima, maxima,
+// compares, selects), at 14 of its instructions a distance with a test of each
+// and XX here: two million clusters 229 us, XX now.
 template <bool SEG>
 __device__ __forceinline__ void nn_pair(const float* box, int stride, const uint32_t* seg, int own, int k0, int k1, int n, int radius,
                                         int& j0, int& j1)
@@ -661,33 +671,114 @@ __device__ __forceinline__ void nn_pair(const float* box, int stride, const uint
     uint2 as = make_uint2(0u, 0u);
     if (SEG)
         as = *reinterpret_cast<const uint2*>(seg + own);
-    float best0 = 0.0f, best1 = 0.0f;
+    float best0 = __int_as_float(0x7F800000), best1 = best0; // infinity
+    int quad0 = -1, quad1 = -1;                              // the four clusters that hold the best, if it is inside the window
     j0 = j1 = -1;
-#pragma unroll (SEG ? 4 : 1) // the block kernel has no registers to spare
-    for (int k = k0; k <= k1; k += 2) {
-        const float2 cx = pair_at(0, k), cy = pair_at(1, k), cz = pair_at(2, k);
-        const float2 dx = pair_at(3, k), dy = pair_at(4, k), dz = pair_at(5, k);
+    // half the surface of the merged box of own + q and k + r
+#define PT_NN_DIST(q, r)                                                                                             \
+    half_area(make_float4(fminf(ax.q, cx.r), fminf(ay.q, cy.r), fminf(az.q, cz.r), 0.0f),                            \
+              make_float4(fmaxf(bx.q, dx.r), fmaxf(by.q, dy.r), fmaxf(bz.q, dz.r), 0.0f))
+#define PT_NN_LOAD(k)                                                                                                \
+    const float2 cx = pair_at(0, k), cy = pair_at(1, k), cz = pair_at(2, k), dx = pair_at(3, k), dy = pair_at(4, k), \
+                 dz = pair_at(5, k);
+#define PT_NN_TRY(q, r, i, j, best, jbest, quad)                                                                     \
+    {                                                                                                                \
+        const float d = PT_NN_DIST(q, r);                                                                            \
+        const int off = (j) - (i);                                                                                   \
+        if (cs.r == as.q && off != 0 && off >= -radius && off <= radius && ((jbest < 0 && quad < 0) || d < best)) {  \
+            best = d;                                                                                                \
+            jbest = (j);                                                                                             \
+            quad = -1;                                                                                               \
+        }                                                                                                            \
+    }
+    auto tested = [&](int k) {
+        PT_NN_LOAD(k)
         uint2 cs = make_uint2(0u, k + 1 < n ? 0u : 1u);
         if (SEG)
             cs = *reinterpret_cast<const uint2*>(seg + k);
-        // half the surface of the merged box of own + q and k + r, and whether it is the best so far
-#define PT_NN_TRY(q, r, i, j, best, jbest)                                                                     \
-    {                                                                                                          \
-        const float ex = fmaxf(bx.q, dx.r) - fminf(ax.q, cx.r), ey = fmaxf(by.q, dy.r) - fminf(ay.q, cy.r),    \
-                    ez = fmaxf(bz.q, dz.r) - fminf(az.q, cz.r);                                                \
-        const float d = ex * ey + ey * ez + ez * ex;                                                           \
-        const int off = (j) - (i);                                                                             \
-        if (cs.r == as.q && off != 0 && off >= -radius && off <= radius && (jbest < 0 || d < best)) {          \
-            best = d;                                                                                          \
-            jbest = (j);                                                                                       \
-        }                                                                                                      \
+        PT_NN_TRY(x, x, own, k, best0, j0, quad0)
+        PT_NN_TRY(x, y, own, k + 1, best0, j0, quad0)
+        PT_NN_TRY(y, x, own + 1, k, best1, j1, quad1)
+        PT_NN_TRY(y, y, own + 1, k + 1, best1, j1, quad1)
+    };
+    const int inner = (radius - 1) & ~1; // both clusters of every pair this far away are in both windows
+    int ka = max(k0, own - inner), kb = min(k1, own + inner);
+    if (SEG) {
+        if (as.x != as.y || seg[k0] != as.x || seg[k1 + 1] != as.x)
+            kb = ka - 2; // another segment's clusters, or none, in the window
+    } else if (kb + 1 >= n)
+        kb -= 2;
+    int k = k0;
+    for (; k < min(ka, k1 + 2); k += 2)
+        tested(k);
+    for (int side = 0; side < 2; side++) {
+        const int end = side == 0 ? min(own - 2, kb) : kb;
+#pragma unroll (SEG ? 2 : 1) // the block kernel has no registers to spare
+        for (; k + 2 <= end; k += 4) {
+            float m0, m1;
+            {
+                PT_NN_LOAD(k)
+                m0 = fminf(PT_NN_DIST(x, x), PT_NN_DIST(x, y));
+                m1 = fminf(PT_NN_DIST(y, x), PT_NN_DIST(y, y));
+            }
+            {
+                PT_NN_LOAD(k + 2)
+                m0 = fminf(m0, fminf(PT_NN_DIST(x, x), PT_NN_DIST(x, y)));
+                m1 = fminf(m1, fminf(PT_NN_DIST(y, x), PT_NN_DIST(y, y)));
+            }
+            if (m0 < best0) {
+                best0 = m0;
+                quad0 = k;
+            }
+            if (m1 < best1) {
+                best1 = m1;
+                quad1 = k;
+            }
+        }
+        // what is left of this side, and the pair itself or the rest
+        const int stop = side == 0 ? min(own, k1) : k1;
+        for (; k <= stop; k += 2)
+            tested(k);
     }
-        PT_NN_TRY(x, x, own, k, best0, j0)
-        PT_NN_TRY(x, y, own, k + 1, best0, j0)
-        PT_NN_TRY(y, x, own + 1, k, best1, j1)
-        PT_NN_TRY(y, y, own + 1, k + 1, best1, j1)
+    // the first of the four that is as near as the best
+    for (int h = 2; h >= 0; h -= 2) {
+        if (quad0 >= 0) {
+            PT_NN_LOAD(quad0 + h)
+            if (!(PT_NN_DIST(x, y) > best0))
+                j0 = quad0 + h + 1;
+            if (!(PT_NN_DIST(x, x) > best0))
+                j0 = quad0 + h;
+        }
+        if (quad1 >= 0) {
+            PT_NN_LOAD(quad1 + h)
+            if (!(PT_NN_DIST(y, y) > best1))
+                j1 = quad1 + h + 1;
+            if (!(PT_NN_DIST(y, x) > best1))
+                j1 = quad1 + h;
+        }
+    }
+    // no distance in range (boxes that overflow): the first in the window, as with a test of each
+    if ((j0 < 0 && own < n) || (j1 < 0 && own + 1 < n)) {
+        const bool first0 = j0 < 0, first1 = j1 < 0;
+        quad0 = quad1 = -1;
+        for (k = k0; k <= k1; k += 2) {
+            PT_NN_LOAD(k)
+            uint2 cs = make_uint2(0u, k + 1 < n ? 0u : 1u);
+            if (SEG)
+                cs = *reinterpret_cast<const uint2*>(seg + k);
+            if (first0) {
+                PT_NN_TRY(x, x, own, k, best0, j0, quad0)
+                PT_NN_TRY(x, y, own, k + 1, best0, j0, quad0)
+            }
+            if (first1) {
+                PT_NN_TRY(y, x, own + 1, k, best1, j1, quad1)
+                PT_NN_TRY(y, y, own + 1, k + 1, best1, j1, quad1)
+            }
+        }
+    }
 #undef PT_NN_TRY
-    }
+#undef PT_NN_LOAD
+#undef PT_NN_DIST
 }
 
 // Nearest neighbours of all live clusters: a block stages its NN_CLUSTERS
@@ -781,7 +872,9 @@ __global__ void k_ploc_merge(Scratch s, int parity, BvhNode* nodes, int node_bas
 }
 
 // First live cluster and live count of each segment (clusters keep their
-// segments' order), and the most of any.
+// segments' order), the most of any, and how many have more than PLOC_SMALL_CAP.
+constexpr uint32_t PLOC_SMALL_CAP = 512, PLOC_BLOCK_CAP = 4096;
+
 __global__ void k_ploc_segments(Scratch s, int parity, uint32_t nseg)
 {
     const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
@@ -806,32 +899,48 @@ __global__ void k_ploc_segments(Scratch s, int parity, uint32_t nseg)
     atomicMax(&s.counters[4], live);
     if (live)
         atomicAdd(&s.counters[5], 1u);
+    if (live > PLOC_SMALL_CAP)
+        atomicAdd(&s.counters[6], 1u);
 }
 
-// Finishes the segments with lo_count < live clusters <= CAP, one block each:
-// the same rounds as above on the segment's clusters in shared memory.  A
-// segment's merges do not depend on the others', so the tree is the one that
-// rounds over all segments would give (only the nodes' numbers differ).  The
-// rounds' launches and scans, at 25 us a round however few clusters were left,
-// took most of the build: 36,000 triangles in 56 meshes and 232 instances 3.2
-// ms, 0.87 ms with this; two million in 64 meshes and 10,256 instances 13.4 and
-// 3.1 ms with the search and bounds above.  While fewer clusters than threads are left, several
-// lanes share a cluster's window.
-template <int THREADS, int CAP>
-__global__ void __launch_bounds__(THREADS) k_ploc_block(Scratch s, int parity, BvhNode* nodes, int node_base, uint32_t lo_count, int radius)
+// Finishes the segments with lo_count < live clusters <= CAP, a cluster of
+// blocks (or one block) each: the same rounds as above on the segment's clusters
+// in shared memory.  A segment's merges do not depend on the others', so the tree
+// is the one that rounds over all segments would give (only the nodes' numbers
+// differ).  The rounds' launches and scans, at 25 us a round however few clusters
+// were left, took most of the build: 36,000 triangles in 56 meshes and 232
+// instances 3.2 ms, two million in 64 meshes and 10,256 instances 13.4 ms.
+//
+// The search, all but the last few rounds of a segment's time, is shared by the
+// cluster's blocks: each searches for its part of the clusters and writes what it
+// found to every block, and all of them then merge and compact their own copies
+// alike.  One block alone took 320 us for 4,096 clusters, XX with eight.  While
+// there are fewer clusters than threads, several lanes share a window; at
+// SOLO_CLUSTERS and below the first block goes on alone.
+constexpr uint32_t SOLO_CLUSTERS = 64;
+
+template <int THREADS, int CAP, bool MULTI>
+__global__ void __launch_bounds__(THREADS) k_ploc_block(Scratch s, int parity, BvhNode* nodes, int node_base, uint32_t lo_count,
+                                                        uint32_t multi_count, int radius)
 {
     constexpr int PER = CAP / THREADS;
-    extern __shared__ __align__(16) float s_box[]; // CAP each of lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, reference, neighbour
+    extern __shared__ __align__(16) float s_box[]; // CAP each of lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, reference, neighbour (two)
     int* s_ref = reinterpret_cast<int*>(s_box + 6 * CAP);
-    int* s_nn = s_ref + CAP;
-    __shared__ uint32_t s_warp[THREADS / 32], s_total, s_rank;
-    const uint32_t m = blockIdx.x;
+    __shared__ uint32_t s_warp[THREADS / 32], s_rank;
+    cg::cluster_group cluster = cg::this_cluster();
+    uint32_t nblocks = MULTI ? cluster.num_blocks() : 1u;
+    const uint32_t rank = MULTI ? cluster.block_rank() : 0u;
+    const uint32_t m = blockIdx.x / nblocks;
     uint32_t n = s.seg_live[m];
     if (n == 0 || n <= lo_count || n > (uint32_t)CAP)
         return;
+    if (n <= multi_count)
+        nblocks = 1;
+    if (rank >= nblocks)
+        return;
     const uint32_t first = s.seg_first[m], tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (n == 1) {
-        if (tid == 0)
+        if (tid == 0 && rank == 0)
             s.seg_root[m] = s.c_ref[parity][first];
         return;
     }
@@ -854,53 +963,76 @@ __global__ void __launch_bounds__(THREADS) k_ploc_block(Scratch s, int parity, B
         s_box[5 * CAP + k] = b.z;
         s_ref[k] = s.c_ref[parity][first + k];
     }
-    __syncthreads();
+    if (MULTI && nblocks > 1)
+        cluster.sync(); // every block of the cluster is up before its memory is written
+    else
+        __syncthreads();
     int node = node_base + (int)(s.counters[2 * parity] + first - s_rank);
     auto box_lo = [&](int k) { return make_float4(s_box[k], s_box[CAP + k], s_box[2 * CAP + k], 0.0f); };
     auto box_hi = [&](int k) { return make_float4(s_box[3 * CAP + k], s_box[4 * CAP + k], s_box[5 * CAP + k], 0.0f); };
-    while (n > 1) { // every round merges at least one pair
-        if (n > THREADS) {
-            const int pad = (radius + 1) & ~1;
-            for (int own = 2 * (int)tid; own < (int)n; own += 2 * THREADS) {
+    const int pad = (radius + 1) & ~1;
+    // Two lists of neighbours: a block may be a round ahead of another that still reads the last round's.
+    for (uint32_t round = 0; n > 1; round++) { // every round merges at least one pair
+        int* s_nn = s_ref + CAP + (round & 1) * CAP;
+        auto found = [&](int i, int j) {
+            if (MULTI && nblocks > 1) {
+                for (uint32_t b = 0; b < nblocks; b++)
+                    cluster.map_shared_rank(s_nn, b)[i] = j;
+            } else
+                s_nn[i] = j;
+        };
+        const uint32_t threads = THREADS * nblocks, me = rank * THREADS + tid;
+        if ((n + 1) / 2 > threads / 2) {
+            for (int own = 2 * (int)me; own < (int)n; own += 2 * (int)threads) {
                 int j0, j1;
                 nn_pair<false>(s_box, CAP, nullptr, own, max(0, own - pad), min(own + pad, ((int)n - 1) & ~1), (int)n, radius, j0, j1);
-                s_nn[own] = j0;
+                found(own, j0);
                 if (own + 1 < (int)n)
-                    s_nn[own + 1] = j1;
+                    found(own + 1, j1);
             }
-        }
-        // lanes per cluster: as many as the block has to spare (a power of two)
-        uint32_t share = 1;
-        while (share < 32 && 2 * share * n <= THREADS)
-            share *= 2;
-        for (uint32_t k = tid; n <= THREADS && k < (n * share + 31) / 32 * 32; k += THREADS) { // whole warps: the shuffles below
-            const int i = (int)(k / share), sub = (int)(k % share);
-            float best = 0.0f;
-            int bj = -1;
-            if (i < (int)n) {
-                const float4 li = box_lo(i), hi_i = box_hi(i);
-                const int j_end = min((int)n - 1, i + radius);
+        } else {
+            // lanes per cluster: as many as the blocks have to spare (a power of two)
+            uint32_t share = 1;
+            while (share < 32 && 2 * share * n <= threads)
+                share *= 2;
+            const uint32_t k = me;
+            if (k < (n * share + 31) / 32 * 32) { // whole warps: the shuffles below
+                const int i = (int)(k / share), sub = (int)(k % share);
+                float best = 0.0f;
+                int bj = -1;
+                if (i < (int)n) {
+                    const float4 li = box_lo(i), hi_i = box_hi(i);
+                    const int j_end = min((int)n - 1, i + radius);
 #pragma unroll 4
-                for (int j = max(0, i - radius) + sub; j <= j_end; j += (int)share) {
-                    const float d = half_area(box_min(li, box_lo(j)), box_max(hi_i, box_hi(j)));
-                    if (j != i && (bj < 0 || d < best)) {
-                        best = d;
-                        bj = j;
+                    for (int j = max(0, i - radius) + sub; j <= j_end; j += (int)share) {
+                        const float d = half_area(box_min(li, box_lo(j)), box_max(hi_i, box_hi(j)));
+                        if (j != i && (bj < 0 || d < best)) {
+                            best = d;
+                            bj = j;
+                        }
                     }
                 }
-            }
-            for (uint32_t o = 1; o < share; o <<= 1) {
-                const float od = __shfl_xor_sync(0xffffffffu, best, o);
-                const int oj = __shfl_xor_sync(0xffffffffu, bj, o);
-                if (oj >= 0 && (bj < 0 || od < best || (od == best && oj < bj))) {
-                    best = od;
-                    bj = oj;
+                for (uint32_t o = 1; o < share; o <<= 1) {
+                    const float od = __shfl_xor_sync(0xffffffffu, best, o);
+                    const int oj = __shfl_xor_sync(0xffffffffu, bj, o);
+                    if (oj >= 0 && (bj < 0 || od < best || (od == best && oj < bj))) {
+                        best = od;
+                        bj = oj;
+                    }
                 }
+                if (sub == 0 && i < (int)n)
+                    found(i, bj);
             }
-            if (sub == 0 && i < (int)n)
-                s_nn[i] = bj;
         }
-        __syncthreads();
+        if (MULTI && nblocks > 1) {
+            cluster.sync();
+            if (n <= SOLO_CLUSTERS) {
+                nblocks = 1; // nothing of another block's memory is touched from here on
+                if (rank != 0)
+                    return;
+            }
+        } else
+            __syncthreads();
         // each thread's own run of clusters
         const uint32_t per = (n + THREADS - 1) / THREADS;
         uint32_t flags = 0, mine = 0; // flags: 2 bits each (survives, merges); mine: merges << 16 | survivors
@@ -926,22 +1058,10 @@ __global__ void __launch_bounds__(THREADS) k_ploc_block(Scratch s, int parity, B
         if (lane == 31)
             s_warp[warp] = sum;
         __syncthreads();
-        if (warp == 0) {
-            const uint32_t v = lane < THREADS / 32 ? s_warp[lane] : 0u;
-            uint32_t w = v;
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t u = __shfl_up_sync(0xffffffffu, w, o);
-                if (lane >= (uint32_t)o)
-                    w += u;
-            }
-            if (lane < THREADS / 32)
-                s_warp[lane] = w - v;
-            if (lane == 31)
-                s_total = w;
-        }
-        __syncthreads();
+        const uint32_t of_warp = lane < THREADS / 32 ? s_warp[lane] : 0u;
+        const uint32_t total = __reduce_add_sync(0xffffffffu, of_warp);
         // the survivors are read before any is overwritten
-        const uint32_t before = s_warp[warp] + sum - mine;
+        const uint32_t before = __reduce_add_sync(0xffffffffu, lane < warp ? of_warp : 0u) + sum - mine;
         float4 lo[PER], hi[PER];
         int ref[PER];
         int id = node + (int)(before >> 16);
@@ -957,7 +1077,8 @@ __global__ void __launch_bounds__(THREADS) k_ploc_block(Scratch s, int parity, B
             if (fl & 2u) {
                 const int j = s_nn[i];
                 const float4 lo_j = box_lo(j), hi_j = box_hi(j);
-                nodes[id] = merged_node(lo[c], hi[c], ref[c], lo_j, hi_j, s_ref[j]);
+                if (rank == 0)
+                    nodes[id] = merged_node(lo[c], hi[c], ref[c], lo_j, hi_j, s_ref[j]);
                 lo[c] = box_min(lo[c], lo_j);
                 hi[c] = box_max(hi[c], hi_j);
                 ref[c] = id++;
@@ -978,14 +1099,13 @@ __global__ void __launch_bounds__(THREADS) k_ploc_block(Scratch s, int parity, B
             s_ref[o] = ref[c];
             o++;
         }
-        const uint32_t total = s_total;
         node += (int)(total >> 16);
         n = total & 0xFFFFu;
         __syncthreads();
         if ((total >> 16) == 0)
             break; // only boxes that are not numbers get here: the root is then any of the clusters
     }
-    if (tid == 0)
+    if (tid == 0 && rank == 0)
         s.seg_root[m] = s_ref[0];
 }
 
@@ -1206,18 +1326,52 @@ bool use_ploc_tlas()
 // has at most PLOC_BLOCK_CAP clusters, then a block per segment.  A round takes
 // about 0.84 of the clusters to the next (0.56 the first), so the host
 // estimates how many are needed and looks at the counters once or twice.
-constexpr uint32_t PLOC_SMALL_CAP = 512, PLOC_BLOCK_CAP = 4096;
-
-template <int THREADS, int CAP>
-cudaError_t launch_ploc_block(const Scratch& s, int parity, uint32_t nseg, BvhNode* nodes, int node_base, uint32_t lo_count, int radius,
-                              cudaStream_t st)
+template <int THREADS, int CAP, bool MULTI>
+cudaError_t launch_ploc_block(const Scratch& s, int parity, uint32_t nseg, BvhNode* nodes, int node_base, uint32_t lo_count,
+                              uint32_t multi_count, uint32_t cluster, int radius, cudaStream_t st)
 {
-    const int bytes = 8 * CAP * (int)sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(k_ploc_block<THREADS, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    const int bytes = 9 * CAP * (int)sizeof(float);
+    cudaError_t e = cudaFuncSetAttribute(k_ploc_block<THREADS, CAP, MULTI>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess)
         return e;
-    k_ploc_block<THREADS, CAP><<<nseg, THREADS, bytes, st>>>(s, parity, nodes, node_base, lo_count, radius);
-    return cudaGetLastError();
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = cluster;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = nseg * cluster;
+    cfg.blockDim = THREADS;
+    cfg.dynamicSmemBytes = bytes;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = MULTI ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k_ploc_block<THREADS, CAP, MULTI>, s, parity, nodes, node_base, lo_count, multi_count, radius);
+}
+
+// After the rounds over all segments: blocks for the small segments and
+// clusters of them for the others.  The clusters are as large as leaves a
+// multiprocessor to each block, and take the small segments along (one block
+// each) where all of them fit: one launch instead of two, one behind the other.
+cudaError_t finish_segments(const Scratch& s, int parity, uint32_t nseg, uint32_t most, uint32_t large, BvhNode* nodes, int node_base,
+                            int radius, cudaStream_t st)
+{
+    int dev = 0, sm_count = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess)
+        return e;
+    const uint32_t sms = (uint32_t)sm_count;
+    if (most <= PLOC_SMALL_CAP || nseg > sms)
+        e = launch_ploc_block<PLOC_SMALL_CAP / 2, PLOC_SMALL_CAP, false>(s, parity, nseg, nodes, node_base, 0u, 0u, 1u, radius, st);
+    if (e != cudaSuccess || most <= PLOC_SMALL_CAP)
+        return e;
+    const uint32_t small = nseg > sms ? 0u : nseg - large;
+    uint32_t cluster = 8;
+    while (cluster > 1 && cluster * large + small > sms)
+        cluster /= 2;
+    return launch_ploc_block<1024, PLOC_BLOCK_CAP, true>(s, parity, nseg, nodes, node_base, nseg > sms ? PLOC_SMALL_CAP : 0u, PLOC_SMALL_CAP,
+                                                         cluster, radius, st);
 }
 
 cudaError_t build_ploc(Scratch& s, uint32_t n, uint32_t nseg, BvhNode* nodes, int node_base, int mode_tlas, cudaStream_t st)
@@ -1230,12 +1384,12 @@ cudaError_t build_ploc(Scratch& s, uint32_t n, uint32_t nseg, BvhNode* nodes, in
         return e;
     const size_t nn_bytes = 7 * sizeof(float) * (size_t)(NN_CLUSTERS + 2 * ((radius + 1) & ~1));
     int parity = 0;
-    uint32_t cap = n, rounds = 0, most = 0;
+    uint32_t cap = n, rounds = 0, most = 0, large = 0;
     for (;;) {
-        if ((e = cudaMemsetAsync(&s.counters[4], 0, 2 * sizeof(uint32_t), st)) != cudaSuccess)
+        if ((e = cudaMemsetAsync(&s.counters[4], 0, 3 * sizeof(uint32_t), st)) != cudaSuccess)
             return e;
         k_ploc_segments<<<blocks(nseg, 128), 128, 0, st>>>(s, parity, nseg);
-        uint32_t c[6];
+        uint32_t c[7];
         e = cudaMemcpyAsync(c, s.counters, sizeof(c), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess)
             e = cudaStreamSynchronize(st);
@@ -1243,6 +1397,7 @@ cudaError_t build_ploc(Scratch& s, uint32_t n, uint32_t nseg, BvhNode* nodes, in
             return e;
         cap = c[2 * parity + 1];
         most = c[4];
+        large = c[6];
         s.blas_nodes = n - c[5]; // a segment of k primitives gets k - 1 nodes
         if (most <= PLOC_BLOCK_CAP)
             break;
@@ -1261,10 +1416,7 @@ cudaError_t build_ploc(Scratch& s, uint32_t n, uint32_t nseg, BvhNode* nodes, in
             parity ^= 1;
         }
     }
-    e = launch_ploc_block<PLOC_SMALL_CAP / 2, PLOC_SMALL_CAP>(s, parity, nseg, nodes, node_base, 0u, radius, st);
-    if (e == cudaSuccess && most > PLOC_SMALL_CAP)
-        e = launch_ploc_block<1024, PLOC_BLOCK_CAP>(s, parity, nseg, nodes, node_base, PLOC_SMALL_CAP, radius, st);
-    return e;
+    return finish_segments(s, parity, nseg, most, large, nodes, node_base, radius, st);
 }
 
 float env_float(const char* name, float dflt)
