@@ -112,7 +112,7 @@ struct Scratch {
     uint64_t* scan;     // exclusive sums of (merge flag << 32 | survivor flag)
     uint32_t* counters; // rounds alternate between two pairs: [2p] nodes emitted, [2p + 1] live clusters at the
                         // start of rounds of parity p; [4] the most live clusters of a segment, [5] segments that
-                        // have any
+                        // have any, [6] segments with more than PLOC_SMALL_CAP
     uint32_t* seg_live; // live clusters of each segment when its block takes over,
     uint32_t* seg_first; // and the first of them
     void* scan_temp;
@@ -659,8 +659,8 @@ __global__ void k_ploc_init(Scratch s, uint32_t n, int mode_tlas)
 // segments' order.  There four clusters are read at a time and only the smallest
 // of their four distances is compared; which of the four it was is found at the
 // end.  The kernels that call it are bound by the ALU pipe (minima, maxima,
-// compares, selects), at 14 of its instructions a distance with a test of each
-// and XX here: two million clusters 229 us, XX now.
+// compares, selects; 80 % busy with a test of each distance): two million
+// clusters 229 us with the tests, 182 without.
 template <bool SEG>
 __device__ __forceinline__ void nn_pair(const float* box, int stride, const uint32_t* seg, int own, int k0, int k1, int n, int radius,
                                         int& j0, int& j1)
@@ -783,7 +783,7 @@ __device__ __forceinline__ void nn_pair(const float* box, int stride, const uint
 
 // Nearest neighbours of all live clusters: a block stages its NN_CLUSTERS
 // clusters and the window on either side.  Bound by the arithmetic of the
-// n (2 radius + 1) distances: two million clusters 230 us (381 with a thread
+// n (2 radius + 1) distances: two million clusters 182 us (381 with a thread
 // to a cluster reading the boxes through L1), 10,000 10 us (29).
 constexpr int NN_THREADS = 128, NN_CLUSTERS = 2 * NN_THREADS;
 
@@ -914,9 +914,11 @@ __global__ void k_ploc_segments(Scratch s, int parity, uint32_t nseg)
 // The search, all but the last few rounds of a segment's time, is shared by the
 // cluster's blocks: each searches for its part of the clusters and writes what it
 // found to every block, and all of them then merge and compact their own copies
-// alike.  One block alone took 320 us for 4,096 clusters, XX with eight.  While
-// there are fewer clusters than threads, several lanes share a window; at
-// SOLO_CLUSTERS and below the first block goes on alone.
+// alike: 10,256 instances, from 4,096 clusters on, 415 us with one block and 179
+// with eight; 44 meshes of 36,000 triangles 323 and 154.  While there are fewer
+// clusters than threads, several lanes share a window; at SOLO_CLUSTERS and below
+// the first block goes on alone.  What is left is the latency of some 50 rounds;
+// more threads or blocks for the small segments changed nothing.
 constexpr uint32_t SOLO_CLUSTERS = 64;
 
 template <int THREADS, int CAP, bool MULTI>
