@@ -270,12 +270,24 @@ __device__ __forceinline__ uint32_t rays_per_fetch(uint32_t count)
     return min(32u, max(1u, (count + warps - 1) / warps));
 }
 
+constexpr int REFILL_KEEP = 12;
+
 // Persistent traversal: warps fetch up to 32 queue entries at a time.
-// Only traces: k_wf_split then separates hits from misses.  A warp's rays end at
-// different steps and their results are written together after the last: written
-// as each one ended, by a lane or two at a time, extend of the mid scene at
-// 1024 x 1024, 128 spp took 50.9 ms against 49.5, and the shadow rays, whose
-// light terms take four loads each, 22.2 against 18.5.
+// Only traces: k_wf_split then separates hits from misses.
+//
+// When all but `keep` of a warp's rays have ended their results are written and
+// their lanes fetch new rays, while the others go on.  Fetching only when all have
+// ended leaves most lanes idle behind the longest ray: heavy scene at 1920 x 1080,
+// 4 spp, extend 20.2 ms against 18.7 and shadow rays 10.5 against 9.0; mid scene at
+// 1024 x 1024, 128 spp, 48.0 both and 18.6 against 16.6.  With 8 kept the whole
+// heavy image takes 29.6 ms and the mid one 79.8, with 12 29.4 and 79.7, with 16
+// 29.3 and 79.8, with 24 28.7 and 80.6.  Not with fewer than 32 rays to a warp,
+// where the queue is empty after the first fetch and the next one only delays the
+// rays that are left (a 160 x 120 preview 583 us, 594 with it).  Fetching for every
+// ray that ends (PT_REFILL=1) is slower than no refill, and so is writing each
+// result as its ray ends, by a lane or two at a time: 50.9 ms of extend on the mid
+// scene against 49.5, and 22.2 ms of shadow rays, whose light terms take four loads
+// each, against 18.5.
 //
 // With a step budget (4-wide nodes, budget > 0) this is the first of two
 // passes: a ray still traversing after `budget` steps is parked (its state
@@ -295,20 +307,30 @@ __global__ void __launch_bounds__(128, TRAV == TRAV_BVH4 ? 8 : 1) k_wf_extend(Wa
     const uint32_t count = *(volatile uint32_t*)&a.w.counts[qi];
     unsigned lane = threadIdx.x & 31;
     const uint32_t take = rays_per_fetch(count);
+    const int keep = BUDGET || take < 32 ? 0 : REFILL_KEEP;
     TraceCounters tc{0u, 0u};
+    const unsigned lower = (1u << lane) - 1u;
+    uint32_t p = 0, job = 0;
+    bool ok = false, live = false; // ok: the lane has a ray whose hit is not written yet; live: it is not finished
+    bool more = true;
+    ClosestTrace t;
+    TraceStack stack;
+    t.ref = REF_DONE;
     while (true) {
-        uint32_t base = 0;
-        if (lane == 0)
-            base = atomicAdd(&a.w.counts[3], take);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= count)
-            break;
-        uint32_t i = base + lane;
-        uint32_t p = 0;
-        bool ok = lane < take && i < count;
-        if (ok) {
-            p = queue[i];
-            PT_CHECK_ENTRY(ok, p, a)
+        const unsigned idle = __ballot_sync(0xffffffffu, !live);
+        if (more) {
+            const uint32_t busy = 32u - (uint32_t)__popc(idle), want = take > busy ? take - busy : 0u;
+            uint32_t base = 0;
+            if (lane == 0)
+                base = atomicAdd(&a.w.counts[3], want);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            more = base + want < count;
+            const uint32_t rank = (uint32_t)__popc(idle & lower);
+            if (!live && rank < want && base + rank < count) {
+                p = queue[base + rank];
+                ok = true;
+                PT_CHECK_ENTRY(ok, p, a)
+            }
         }
         if (TRAV == TRAV_BVH2_WW) {
             if (ok) {
@@ -318,20 +340,21 @@ __global__ void __launch_bounds__(128, TRAV == TRAV_BVH4 ? 8 : 1) k_wf_extend(Wa
                 const bool hit = trace_closest_ww(s, mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), o.w, d.w, h, tc);
                 a.w.hit[p] = make_float4(h.t, h.b1, h.b2, __uint_as_float(h.inst));
                 a.w.hit_prim[p] = hit ? h.prim : 0xFFFFFFFFu;
+                ok = false;
             }
+            if (!more)
+                break;
             continue;
+        }
+        if (ok && !live) {
+            job = a.src.job_of(p);
+            const float4 o = a.w.ray_o[p], d = a.w.ray_d[p];
+            closest_begin(a.src.args(job).s, mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), o.w, d.w, t, stack);
+            live = true;
         }
         // one warp-uniform loop (a single copy of the step code): with a step
         // budget, the lanes still traversing at iteration `budget` park together
-        ClosestTrace t;
-        TraceStack stack;
-        t.ref = REF_DONE;
-        const DevScene& s = a.src.args(ok ? a.src.job_of(p) : 0u).s;
-        bool live = ok;
-        if (ok) {
-            const float4 o = a.w.ray_o[p], d = a.w.ray_d[p];
-            closest_begin(s, mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), o.w, d.w, t, stack);
-        }
+        const DevScene& s = a.src.args(job).s;
         for (uint32_t k = 0;; k++) {
             if (BUDGET && k == budget) {
                 const bool park = live && t.sp <= PARK_STACK;
@@ -349,15 +372,18 @@ __global__ void __launch_bounds__(128, TRAV == TRAV_BVH4 ? 8 : 1) k_wf_extend(Wa
                     }
                 }
             }
-            if (!__any_sync(0xffffffffu, live))
+            if (__popc(__ballot_sync(0xffffffffu, live)) <= (more ? keep : 0))
                 break;
             if (closest_step_warp<TRAV == TRAV_BVH4>(s, live, t, stack, tc))
                 live = false;
         }
-        if (ok) {
+        if (ok && !live) {
             a.w.hit[p] = make_float4(t.h.t, t.h.b1, t.h.b2, __uint_as_float(t.h.inst));
             a.w.hit_prim[p] = t.found ? t.h.prim : 0xFFFFFFFFu;
+            ok = false;
         }
+        if (!more)
+            break;
     }
     uint32_t nodes = __reduce_add_sync(0xffffffffu, tc.nodes);
     uint32_t tris = __reduce_add_sync(0xffffffffu, tc.tris);
@@ -744,27 +770,37 @@ __global__ void __launch_bounds__(128, W4 ? 8 : 1) k_wf_shadow(WaveArgs<Src> a, 
     const uint32_t count = a.w.counts[2];
     unsigned lane = threadIdx.x & 31;
     const uint32_t take = rays_per_fetch(count);
+    const int keep = BUDGET || take < 32 ? 0 : REFILL_KEEP;
     TraceCounters tc{0u, 0u};
+    const unsigned lower = (1u << lane) - 1u;
+    uint32_t p = 0, job = 0;
+    bool ok = false, live = false, more = true; // ok, live and the refill as in k_wf_extend
+    ShadowTrace t;
+    TraceStack stack;
+    t.ref = REF_DONE;
     while (true) {
-        uint32_t base = 0;
-        if (lane == 0)
-            base = atomicAdd(&a.w.counts[4], take);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= count)
-            break;
-        uint32_t i = base + lane;
-        bool ok = lane < take && i < count;
-        uint32_t p = ok ? a.w.shadow_queue[i] : 0u;
-        PT_CHECK_ENTRY(ok, p, a)
-        ShadowTrace t;
-        TraceStack stack;
-        t.ref = REF_DONE;
-        const DevScene& s = a.src.args(ok ? a.src.job_of(p) : 0u).s;
-        bool live = ok;
-        if (ok) {
-            const float4 o = a.w.nee_o[p], d = a.w.nee_d[p];
-            shadow_begin(s, mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), 0.0f, o.w, t, stack);
+        const unsigned idle = __ballot_sync(0xffffffffu, !live);
+        if (more) {
+            const uint32_t busy = 32u - (uint32_t)__popc(idle), want = take > busy ? take - busy : 0u;
+            uint32_t base = 0;
+            if (lane == 0)
+                base = atomicAdd(&a.w.counts[4], want);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            more = base + want < count;
+            const uint32_t rank = (uint32_t)__popc(idle & lower);
+            if (!live && rank < want && base + rank < count) {
+                p = a.w.shadow_queue[base + rank];
+                ok = true;
+                PT_CHECK_ENTRY(ok, p, a)
+            }
         }
+        if (ok && !live) {
+            job = a.src.job_of(p);
+            const float4 o = a.w.nee_o[p], d = a.w.nee_d[p];
+            shadow_begin(a.src.args(job).s, mk3(o.x, o.y, o.z), mk3(d.x, d.y, d.z), 0.0f, o.w, t, stack);
+            live = true;
+        }
+        const DevScene& s = a.src.args(job).s;
         for (uint32_t k = 0;; k++) {
             if (BUDGET && k == budget) {
                 const bool park = live && t.sp <= PARK_STACK;
@@ -782,13 +818,17 @@ __global__ void __launch_bounds__(128, W4 ? 8 : 1) k_wf_shadow(WaveArgs<Src> a, 
                     }
                 }
             }
-            if (!__any_sync(0xffffffffu, live))
+            if (__popc(__ballot_sync(0xffffffffu, live)) <= (more ? keep : 0))
                 break;
             if (shadow_step_warp<W4>(s, live, t, stack, tc))
                 live = false;
         }
-        if (ok)
+        if (ok && !live) {
             shadow_finish(a, p, shadow_result(t));
+            ok = false;
+        }
+        if (!more)
+            break;
     }
     uint32_t nodes = __reduce_add_sync(0xffffffffu, tc.nodes);
     uint32_t tris = __reduce_add_sync(0xffffffffu, tc.tris);
