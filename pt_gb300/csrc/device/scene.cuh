@@ -419,6 +419,11 @@ constexpr int STACK_SIZE = 96;
 // any-hit queries whose result does not depend on the order).  Returns false
 // when no child was hit (the caller pops).  A push that would overflow sets
 // ERR_STACK_OVERFLOW and drops those children.
+// All lanes with a hit go the same way, whatever their number of hits: a way of
+// its own for one hit, and a loop over the other hits of an any-hit step, cost a
+// warp both ways on nearly every step (mid scene at 1024 x 1024, 128 spp, extend
+// 48.4 -> 47.5 ms, shadow rays 16.6 -> 15.1; heavy scene at 1920 x 1080, 4 spp
+// 18.9 -> 18.4 and 8.9 -> 8.1).
 template <bool SORT, class Stack>
 __device__ __forceinline__ bool step4(const DevScene& s, const ObjRay& r, float tmin, float tmax, int& ref, Stack& stack, int& sp)
 {
@@ -426,22 +431,22 @@ __device__ __forceinline__ bool step4(const DevScene& s, const ObjRay& r, float 
     int c[4];
     const int m = node4_children(s.nodes4 + ref, r, tmin, tmax, e, c);
     const int cnt = __popc(m);
-    if (cnt == 0)
-        return false;
-    if (cnt == 1) {
-        ref = c[__ffs(m) - 1];
-        return true;
-    }
     if (!SORT) {
-        ref = c[__ffs(m) - 1];
+        ref = (m & 1) ? c[0] : (m & 2) ? c[1] : (m & 4) ? c[2] : c[3];
         if (sp + cnt - 1 > STACK_SIZE) {
             atomicOr(s.error_word, ERR_STACK_OVERFLOW);
             return true;
         }
-        for (int rest = m & (m - 1); rest; rest &= rest - 1)
-            stack.set(sp++, c[__ffs(rest) - 1]);
-        return true;
+        if ((m & 2) && (m & 1))
+            stack.set(sp++, c[1]);
+        if ((m & 4) && (m & 3))
+            stack.set(sp++, c[2]);
+        if ((m & 8) && (m & 7))
+            stack.set(sp++, c[3]);
+        return cnt != 0;
     }
+    if (cnt == 0)
+        return false;
     // sort (entry, child) ascending with misses keyed +inf: a five-exchange network
     const float inf = __int_as_float(0x7f800000);
     float k0 = (m & 1) ? e[0] : inf, k1 = (m & 2) ? e[1] : inf, k2 = (m & 4) ? e[2] : inf, k3 = (m & 8) ? e[3] : inf;
@@ -468,7 +473,8 @@ __device__ __forceinline__ bool step4(const DevScene& s, const ObjRay& r, float 
             stack.set(sp++, r3);
         if (cnt >= 3)
             stack.set(sp++, r2);
-        stack.set(sp++, r1);
+        if (cnt >= 2)
+            stack.set(sp++, r1);
     }
     ref = r0;
     return true;
