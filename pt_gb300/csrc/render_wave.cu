@@ -1036,11 +1036,12 @@ struct StageVariant {
     int shade = 6;       // resident-block target of shade (0: none)
     uint32_t refill = 0; // 0: no refill; else 1..32
     uint32_t budget = 48; // extend's first-pass step budget over 4-wide nodes (PT_EXTEND_BUDGET; 0: one pass)
-    // two passes only for waves of at least 2^budget_min_log2 paths
-    // (PT_EXTEND_BUDGET_MIN_LOG2): smaller waves ran 2-11 % faster in one
-    // pass (the resume launch's latency tail), waves of 2^25 paths and more
-    // 0.3-0.5 % slower
-    uint32_t budget_min_log2 = 25;
+    // Two passes for waves of at least 2^budget_min_log2 paths
+    // (PT_EXTEND_BUDGET_MIN_LOG2; 32: none).  Parking was 0.3-0.5 % faster on
+    // waves of 2^25 paths and more while a warp waited for its longest ray; since
+    // warps refill, the mid scene at 1024 x 1024, 128 spp takes 77.8 ms with it
+    // and 75.9 in one pass (extend 47.5 and 45.1).
+    uint32_t budget_min_log2 = 32;
     uint32_t shadow_budget = 0; // the same for shadow rays (PT_SHADOW_BUDGET; measured slower, off)
 };
 

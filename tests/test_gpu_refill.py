@@ -1,7 +1,14 @@
 """Traversal warps that fetch new rays while some of theirs go on (GPU): images
 and traversal counts equal those of the megakernel, which traces every ray by
 itself, for queues below, at and above the size from which warps do so, with and
-without transparent instances.  No tolerance: every ray takes the same steps."""
+without transparent instances.  Extend refills in one pass only, so the same
+comparison also runs in a process without the step budget that the other tests
+set.  No tolerance: every ray takes the same steps."""
+import os
+import subprocess
+import sys
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -34,10 +41,7 @@ def _scene(alpha):
     return P.HostScene.from_raw(scenes.assemble_raw(meshes, (0.1, 0.15, 0.3)), cam)
 
 
-# 152 x 32 resident warps, half of them counted, 32 rays each: warps are refilled from 77,793 rays on
-@pytest.mark.parametrize("alpha", [False, True])
-@pytest.mark.parametrize("w,h,spp", [(61, 37, 1), (304, 255, 1), (305, 256, 1), (509, 333, 3)])
-def test_wavefront_equals_megakernel(w, h, spp, alpha):
+def _check(w, h, spp, alpha):
     hs = _scene(alpha)
     with P.Context(0) as ctx:
         ctx.upload(hs.pack())
@@ -46,3 +50,21 @@ def test_wavefront_equals_megakernel(w, h, spp, alpha):
         got, got_counts = _render(ctx, hs, w, h, spp, abi.PT_KERNEL_WAVEFRONT)
     assert counts == got_counts
     assert np.array_equal(img.view(np.uint32), got.view(np.uint32))
+
+
+# 152 x 32 resident warps, half of them counted, 32 rays each: warps are refilled from 75,393 rays on
+SIZES = [(61, 37, 1), (304, 247, 1), (305, 248, 1), (509, 333, 3)]
+
+
+@pytest.mark.parametrize("alpha", [False, True])
+@pytest.mark.parametrize("w,h,spp", SIZES)
+def test_wavefront_equals_megakernel(w, h, spp, alpha):
+    _check(w, h, spp, alpha)
+
+
+@pytest.mark.parametrize("alpha", [False, True])
+def test_one_pass_equals_megakernel(alpha):
+    root = Path(__file__).resolve().parent.parent
+    code = f"import sys; sys.path[:0] = ['tests', '.']; import test_gpu_refill as t; [t._check(w, h, s, {alpha}) for w, h, s in t.SIZES]"
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, PT_EXTEND_BUDGET="0"), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
