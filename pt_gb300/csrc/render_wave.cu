@@ -279,9 +279,9 @@ constexpr int REFILL_KEEP = 12;
 // their lanes fetch new rays, while the others go on.  Fetching only when all have
 // ended leaves most lanes idle behind the longest ray: heavy scene at 1920 x 1080,
 // 4 spp, extend 20.2 ms against 18.7 and shadow rays 10.5 against 9.0; mid scene at
-// 1024 x 1024, 128 spp, 48.0 both and 18.6 against 16.6.  With 8 kept the whole
-// heavy image takes 29.6 ms and the mid one 79.8, with 12 29.4 and 79.7, with 16
-// 29.3 and 79.8, with 24 28.7 and 80.6.  Not with fewer than 32 rays to a warp,
+// 1024 x 1024, 128 spp, 47.5 against 45.1 and 18.6 against 16.6.  With 8 kept the
+// whole heavy image takes 28.4 ms and the mid one 76.1, with 12 28.3 and 76.1, with
+// 16 27.9 and 76.8, with 20 27.6 and 78.0.  Not with fewer than 32 rays to a warp,
 // where the queue is empty after the first fetch and the next one only delays the
 // rays that are left (a 160 x 120 preview 583 us, 594 with it).  Fetching for every
 // ray that ends (PT_REFILL=1) is slower than no refill, and so is writing each
