@@ -297,9 +297,10 @@ constexpr int REFILL_KEEP = 12;
 // is deeper than PARK_STACK, or that finds no free slot, finishes here.  The
 // hit is the same either way: the resumed traversal continues the same
 // sequence of steps.
-// Residency: 8 blocks of 128 per SM (64 registers, 32-40 B of spills) over
-// the half-precision 4-wide nodes; on the heavy scene 7 blocks measured 25.2
-// against 24.5 ms of extend (on the mid scene 58.9 and 58.7).
+// Residency: 8 blocks of 128 per SM (64 registers, 22-40 B of spills) over
+// the half-precision 4-wide nodes: heavy scene at 1920 x 1080, 4 spp, extend
+// 18.4 ms (19.5 at 7 blocks, 18.1 at 9), mid scene at 1024 x 1024, 128 spp 47.5
+// (49.5 and 48.5).
 template <class Src, int TRAV, bool BUDGET = false>
 __global__ void __launch_bounds__(128, TRAV == TRAV_BVH4 ? 8 : 1) k_wf_extend(WaveArgs<Src> a, uint32_t qi, uint32_t budget)
 {
@@ -759,8 +760,8 @@ __device__ __forceinline__ void shadow_finish(const WaveArgs<Src>& a, uint32_t p
     a.w.rad[p] = make_float4(rad.x, rad.y, rad.z, 0.0f);
 }
 
-// Persistent shadow (any-hit) traversal, 8 blocks of 128 per SM (on the heavy
-// scene 12.44 ms of shadow against 12.84 at 7).  With BUDGET (4-wide nodes) the
+// Persistent shadow (any-hit) traversal, 8 blocks of 128 per SM (heavy scene 8.2
+// ms of shadow rays against 8.6 at 7, mid scene 15.1 against 15.8).  With BUDGET (4-wide nodes) the
 // first of two passes, as k_wf_extend: rays still traversing after `budget`
 // steps park (counters [8]/[9]) and k_wf_shadow_resume finishes them.
 template <class Src, bool W4, bool BUDGET = false>
