@@ -241,10 +241,22 @@ struct ObjRay {
 constexpr uint32_t SLAB_HI_X = 1u, SLAB_HI_Y = 2u, SLAB_HI_Z = 4u;
 constexpr uint32_t AXIS_X_IS_1 = 8u, AXIS_X_IS_2 = 16u, AXIS_Y_IS_1 = 32u, AXIS_Y_IS_2 = 64u, AXIS_Z_IS_1 = 128u, AXIS_Z_IS_2 = 256u;
 
-__device__ __forceinline__ void setup_slab(ObjRay& r)
+// Shadow rays without an end lead to directional lights, and one along an axis
+// makes every one of them a ray with zero components: they take the finite
+// inverses (slab.h), without which they lost every node across a coordinate
+// plane.  Any other ray has a component of exactly zero by chance only, about
+// once in 10^8, and keeps 1 / d: of the mid scene at 1024 x 1024, 128 spp, two
+// pixels would differ (they miss a hit that the oracle finds) and every ray and
+// instance entry would pay for it (83.3 -> 84.6 ms).
+__device__ __forceinline__ void setup_slab(ObjRay& r, bool endless)
 {
     r.inv_d = mk3(1.0f / r.d.x, 1.0f / r.d.y, 1.0f / r.d.z);
     r.o_inv = mk3(r.o.x * r.inv_d.x, r.o.y * r.inv_d.y, r.o.z * r.inv_d.z);
+    if (endless) {
+        slab_finite(r.o.x, r.inv_d.x, r.o_inv.x);
+        slab_finite(r.o.y, r.inv_d.y, r.o_inv.y);
+        slab_finite(r.o.z, r.inv_d.z, r.o_inv.z);
+    }
     r.axes = (slab_hi_first(__float_as_uint(r.inv_d.x)) ? SLAB_HI_X : 0u) | (slab_hi_first(__float_as_uint(r.inv_d.y)) ? SLAB_HI_Y : 0u) |
              (slab_hi_first(__float_as_uint(r.inv_d.z)) ? SLAB_HI_Z : 0u);
 }
@@ -279,8 +291,8 @@ __device__ __forceinline__ void setup_watertight(ObjRay& r)
 }
 
 // Robust slab test (Ize 2013): far distances are scaled by 1 + 2*gamma(3).
-// Box planes are padded at build time, so NaNs from 0*inf (a ray on a slab
-// plane of a zero direction component) are ignored by fminf/fmaxf safely.
+// NaN distances (an infinite inverse of a zero direction component) are ignored
+// by fminf / fmaxf; what that misses is said at setup_slab.
 constexpr float SLAB_SCALE = 1.0f + 2.0f * (3.0f * 0x1p-24f) / (1.0f - 3.0f * 0x1p-24f);
 
 __device__ __forceinline__ float slab_enter(float lo, float hi, float inv, float oinv, float& tfar)
@@ -515,13 +527,13 @@ __device__ __forceinline__ bool watertight(const ObjRay& r, f3 p0, f3 p1, f3 p2,
     return true;
 }
 
-__device__ __forceinline__ void to_object(const DevInstance* di, f3 o, f3 d, ObjRay& r)
+__device__ __forceinline__ void to_object(const DevInstance* di, f3 o, f3 d, ObjRay& r, bool endless)
 {
     float4 w0 = ldg4(&di->w2o[0]), w1 = ldg4(&di->w2o[1]), w2 = ldg4(&di->w2o[2]);
     r.o = mk3(((w0.x * o.x + w0.y * o.y) + w0.z * o.z) + w0.w, ((w1.x * o.x + w1.y * o.y) + w1.z * o.z) + w1.w,
               ((w2.x * o.x + w2.y * o.y) + w2.z * o.z) + w2.w);
     r.d = mk3((w0.x * d.x + w0.y * d.y) + w0.z * d.z, (w1.x * d.x + w1.y * d.y) + w1.z * d.z, (w2.x * d.x + w2.y * d.y) + w2.z * d.z);
-    setup_slab(r);
+    setup_slab(r, endless);
     setup_watertight(r);
 }
 
@@ -606,7 +618,7 @@ __device__ __forceinline__ void closest_begin(const DevScene& s, f3 o, f3 d, flo
     t.found = false;
     t.world.o = o;
     t.world.d = d;
-    setup_slab(t.world);
+    setup_slab(t.world, false);
     t.r = t.world;
     t.tmin = tmin;
     t.sp = 0;
@@ -669,7 +681,7 @@ __device__ __forceinline__ bool closest_leaf(const DevScene& s, ClosestTrace& t,
             atomicOr(s.error_word, ERR_STACK_OVERFLOW);
             return true;
         }
-        to_object(di, t.world.o, t.world.d, t.r);
+        to_object(di, t.world.o, t.world.d, t.r, false);
         stack.set(t.sp++, REF_EXIT_BLAS);
         t.in_blas = true;
         t.ref = root;
@@ -753,7 +765,7 @@ __device__ __forceinline__ void resume_closest(const DevScene& s, const TracePar
     const float4 h = pk.hit[slot];
     t.world.o = o;
     t.world.d = d;
-    setup_slab(t.world);
+    setup_slab(t.world, false);
     t.tmin = tmin;
     t.ref = st.x;
     t.sp = st.y & 0xFFFF;
@@ -767,7 +779,7 @@ __device__ __forceinline__ void resume_closest(const DevScene& s, const TracePar
     t.h.inst = __float_as_uint(h.w);
     t.h.prim = pk.prim[slot];
     if (t.in_blas)
-        to_object(s.dinst + t.cur_inst, t.world.o, t.world.d, t.r);
+        to_object(s.dinst + t.cur_inst, t.world.o, t.world.d, t.r, false);
     else
         t.r = t.world;
     for (int k = 0; k < t.sp; k++)
@@ -807,7 +819,7 @@ static __device__ __forceinline__ bool trace_closest_ww(const DevScene& s, f3 o,
     ObjRay world;
     world.o = o;
     world.d = d;
-    setup_slab(world);
+    setup_slab(world, false);
     ObjRay r = world;
     int stack[STACK_SIZE];
     int sp = 0;
@@ -864,7 +876,7 @@ static __device__ __forceinline__ bool trace_closest_ww(const DevScene& s, f3 o,
                     ref = stack[--sp];
                 } else {
                     cur_inst = first;
-                    to_object(di, o, d, r);
+                    to_object(di, o, d, r, false);
                     stack[sp++] = REF_EXIT_BLAS;
                     in_blas = true;
                     ref = root;
@@ -926,11 +938,14 @@ struct ShadowTrace {
     bool in_blas, opaque, alpha_map; // alpha_map: the transparent instance's alpha comes from a base colour map
 };
 
+// A shadow ray to a directional light (setup_slab).
+__device__ __forceinline__ bool endless(float tmax) { return tmax > 3.402823466e38f; }
+
 __device__ __forceinline__ void shadow_begin(const DevScene& s, f3 o, f3 d, float tmin, float tmax, ShadowTrace& t, TraceStack& stack)
 {
     t.world.o = o;
     t.world.d = d;
-    setup_slab(t.world);
+    setup_slab(t.world, endless(tmax));
     t.r = t.world;
     t.tmin = tmin;
     t.tmax = tmax;
@@ -987,7 +1002,7 @@ __device__ __forceinline__ bool shadow_leaf(const DevScene& s, ShadowTrace& t, T
             atomicOr(s.error_word, ERR_STACK_OVERFLOW);
             return true;
         }
-        to_object(di, t.world.o, t.world.d, t.r);
+        to_object(di, t.world.o, t.world.d, t.r, endless(t.tmax));
         stack.set(t.sp++, REF_EXIT_BLAS);
         t.in_blas = true;
         t.ref = root;
@@ -1093,7 +1108,7 @@ __device__ __forceinline__ void resume_shadow(const DevScene& s, const TracePark
     const float4 h = pk.hit[slot];
     t.world.o = o;
     t.world.d = d;
-    setup_slab(t.world);
+    setup_slab(t.world, endless(tmax));
     t.tmin = tmin;
     t.tmax = tmax;
     t.ref = st.x;
@@ -1108,7 +1123,7 @@ __device__ __forceinline__ void resume_shadow(const DevScene& s, const TracePark
     t.alpha_pass = h.y;
     t.alpha_tex = __float_as_uint(h.z);
     if (t.in_blas)
-        to_object(s.dinst + t.inst, t.world.o, t.world.d, t.r);
+        to_object(s.dinst + t.inst, t.world.o, t.world.d, t.r, endless(t.tmax));
     else
         t.r = t.world;
     for (int k = 0; k < t.sp; k++)
