@@ -550,15 +550,20 @@ cudaError_t conv3x3_wgrad(const WgradCall& c, int sm_count, uint32_t* error, cud
     const size_t tail = (size_t)(16 - 3 * p.nc) * p.row_bytes + 128 + 8 * (2 * 4 + 1) + 32;
     size_t stage = 0;
     // the most rows to a chunk (an input row is loaded (ry + 2) / ry times) that leave two stages, then as many
-    // stages as fit
-    for (p.ry = 8; p.ry >= 1; p.ry /= 2) {
-        stage = (size_t)p.tiles_per_cta * (p.ry + 2) * p.nc * p.row_bytes + (size_t)(c.cout / 8) * p.ry * p.g_row_bytes;
-        const int loads = p.tiles_per_cta * p.nc * (p.ry + 2) + c.cout / 8 * p.ry;
-        if ((p.ry == 1 || p.ry < 2 * c.h) && 2 * stage + tail <= SMEM_LIMIT && loads <= 32 * WGRAD_LANE_LOADS)
+    // stages as fit; where not even one row does (16 output channels and 288 input channels or more), half of the
+    // tiles to a CTA
+    for (;; p.tiles_per_cta /= 2) {
+        for (p.ry = 8; p.ry >= 1; p.ry /= 2) {
+            stage = (size_t)p.tiles_per_cta * (p.ry + 2) * p.nc * p.row_bytes + (size_t)(c.cout / 8) * p.ry * p.g_row_bytes;
+            const int loads = p.tiles_per_cta * p.nc * (p.ry + 2) + c.cout / 8 * p.ry;
+            if ((p.ry == 1 || p.ry < 2 * c.h) && 2 * stage + tail <= SMEM_LIMIT && loads <= 32 * WGRAD_LANE_LOADS)
+                break;
+        }
+        if (p.ry >= 1)
             break;
+        if (p.tiles_per_cta == 1)
+            return cudaErrorInvalidValue;
     }
-    if (p.ry < 1)
-        return cudaErrorInvalidValue;
     p.stages = (int)std::min<size_t>(4, (SMEM_LIMIT - tail) / stage);
     p.chunks_x = (p.w + p.tx - 1) / p.tx;
     p.chunks_y = (p.h + p.ry - 1) / p.ry;
