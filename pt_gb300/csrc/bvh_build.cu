@@ -39,6 +39,7 @@
 #include <cstring>
 
 #include "device/scene.cuh"
+#include "device/warps.h"
 #include "kernels.h"
 
 namespace pt {
@@ -361,7 +362,7 @@ __device__ __forceinline__ void widen_by_row(float4 row, float4 c, float4 h, flo
 __global__ void __launch_bounds__(BOUNDS_THREADS) k_inst_boxes(BvhBuildInput in, const int* mesh_box, const int* mesh_root,
                                                                const BvhNode* nodes, Scratch s)
 {
-    const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    const uint32_t i = warp_item(blockIdx.x, BOUNDS_THREADS, threadIdx.x), lane = threadIdx.x & 31;
     const bool valid = i < in.instance_count && lane == 0;
     const float inf = __int_as_float(0x7f800000);
     float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
