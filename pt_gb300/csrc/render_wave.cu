@@ -964,8 +964,11 @@ __global__ void __launch_bounds__(256) k_wf_accumulate(WaveArgs<Src> a)
         atomicAdd(a.src.counters() + 2, (unsigned long long)a.src.n_paths);
 }
 
-// Parking slots for a quarter of a wave's paths (a multiple of 32).
-static inline size_t park_slots(size_t n_paths) { return ((n_paths / 4) + 31) / 32 * 32; }
+// Parking slots for a quarter of a wave's paths (a multiple of 32), where the
+// process parks at all: they take 42 of 274 bytes a path, 2.8 GB of a state of
+// 2^26 paths.
+static bool parks();
+static inline size_t park_slots(size_t n_paths) { return parks() ? ((n_paths / 4) + 31) / 32 * 32 : 0; }
 
 size_t wave_state_bytes(uint32_t n_paths)
 {
@@ -1075,6 +1078,13 @@ static StageVariant stage_variant()
         return r;
     }();
     return v;
+}
+
+// Whether any wave's traversal may have a step budget.
+static bool parks()
+{
+    const StageVariant v = stage_variant();
+    return (v.budget && v.budget_min_log2 < 32) || v.shadow_budget;
 }
 
 template <typename K>
