@@ -25,9 +25,10 @@
 // globally closest pair in each segment is always mutual), mutual nearest
 // neighbours merge into a new node, and the survivors are compacted in
 // order, until each segment is one cluster.  Rounds over all segments at once
-// run until every segment is small; then one block per segment finishes it in
-// shared memory.  Nodes are numbered in merge order by prefix sums
-// (deterministic).  PT_BVH=lbvh selects the radix tree instead (kept for A/B).
+// run until every segment is small; then a block or a cluster of blocks per
+// segment finishes it in shared memory.  Nodes are numbered in merge order by
+// prefix sums (deterministic).  PT_BVH=lbvh selects the radix tree instead (kept
+// for A/B).
 #include <cooperative_groups.h>
 #include <cub/cub.cuh>
 #include <thrust/iterator/counting_iterator.h>
@@ -1325,10 +1326,7 @@ bool use_ploc_tlas()
     return v;
 }
 
-// PLOC over the sorted primitives: rounds over all segments until the largest
-// has at most PLOC_BLOCK_CAP clusters, then a block per segment.  A round takes
-// about 0.84 of the clusters to the next (0.56 the first), so the host
-// estimates how many are needed and looks at the counters once or twice.
+// k_ploc_block, `cluster` blocks to a segment (MULTI).
 template <int THREADS, int CAP, bool MULTI>
 cudaError_t launch_ploc_block(const Scratch& s, int parity, uint32_t nseg, BvhNode* nodes, int node_base, uint32_t lo_count,
                               uint32_t multi_count, uint32_t cluster, int radius, cudaStream_t st)
@@ -1377,6 +1375,10 @@ cudaError_t finish_segments(const Scratch& s, int parity, uint32_t nseg, uint32_
                                                          cluster, radius, st);
 }
 
+// PLOC over the sorted primitives: rounds over all segments until the largest
+// has at most PLOC_BLOCK_CAP clusters, then finish_segments.  A round takes
+// about 0.84 of the clusters to the next (0.56 the first), so the host
+// estimates how many are needed and looks at the counters once or twice.
 cudaError_t build_ploc(Scratch& s, uint32_t n, uint32_t nseg, BvhNode* nodes, int node_base, int mode_tlas, cudaStream_t st)
 {
     const int radius = ploc_radius(mode_tlas);

@@ -15,8 +15,8 @@
 //   tris       TriRec, 48 B: the three object-space vertices of a triangle in
 //              BVH leaf order plus its mesh-local primitive index
 //   dinst      DevInstance, 64 B: world-to-object rows + BLAS root reference
-// Traversal reads nodes/tris/dinst with 16-byte vector loads through the
-// read-only path.
+// Traversal reads nodes4 with 32-byte and nodes/tris/dinst with 16-byte vector
+// loads through the read-only path.
 #pragma once
 #include <cstdint>
 #include <cuda_fp16.h>
@@ -29,7 +29,7 @@ namespace pt {
 
 // Child / root reference: >= 0 interior node index; < 0 a leaf holding the
 // primitives (first, count) encoded as ~((first << 2) | (count - 1)), with
-// first < 2^28.  Two sentinels below the leaf range drive the traversal loop.
+// first < 2^28.  Three sentinels below the leaf range drive the traversal loop.
 constexpr int REF_DONE = (int)0x80000000;
 constexpr int REF_EXIT_BLAS = (int)0x80000001;
 constexpr int REF_EMPTY = (int)0x80000002;

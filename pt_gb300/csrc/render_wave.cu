@@ -442,8 +442,9 @@ __global__ void __launch_bounds__(128, 8) k_wf_extend_resume(WaveArgs<Src> a)
 // (pathtrace.ms.hlsl:6-11: radiance += throughput * envcol, the path ends;
 // a camera ray that escapes has zero first-hit features), hits go to the hit
 // queue, so shade runs on hit paths only.  One atomic per block of 256 paths.
-// The previous segment's shadow stage ran before this segment's extend, so
-// the radiance terms keep the reference's order.
+// The previous segment's shadow stage runs beside this segment's extend; this
+// kernel is launched behind a wait for it, so the radiance terms keep the
+// reference's order.
 template <class Src>
 __global__ void __launch_bounds__(256) k_wf_split(WaveArgs<Src> a, uint32_t qi)
 {
@@ -1031,7 +1032,8 @@ static inline uint32_t capped_grid(uint64_t threads, uint32_t block, int sm_coun
 // with PT_TRAVERSAL=ww: on the mid scene the latter ran 24 % slower, its
 // extra node visits and triangle tests costing more than the coherence
 // gained), the per-lane refill of the traversal kernels (PT_REFILL = idle
-// lanes that trigger a fetch, 1-32; 0 = whole-warp fetches of 32 rays) and
+// lanes that trigger a fetch, 1-32; 0 = the kernels without it, whose warps
+// fetch when REFILL_KEEP of their rays are left) and
 // the resident-block target of shade (PT_MINB=5 or 6, 0 for none; default 6:
 // 0.45 % faster than the 4 blocks its natural register count gives, 5
 // blocks slower).  The alternatives stay for A/B measurements.
